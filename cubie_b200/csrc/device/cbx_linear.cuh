@@ -27,7 +27,7 @@ namespace cbx {
 // preconditioner application per iteration, x and r updated with
 // alpha = <t,r>/<t,t> (MR) or <r,z>/<t,z> (SD).  ``rhs`` is overwritten
 // with the running residual and ``x`` holds the initial guess on entry.
-template <class Cfg, class Op, bool SD>
+template <class Cfg, class Op, bool SD, bool ZERO_GUESS>
 __device__ __forceinline__ int solve_mr(const Op& op, typename Cfg::R* rhs,
                                         typename Cfg::R* x, int& iters) {
     using R = typename Cfg::R;
@@ -38,10 +38,13 @@ __device__ __forceinline__ int solve_mr(const Op& op, typename Cfg::R* rhs,
     const C tol2 = tol * tol;
     R z[K];
     R tmp[K];
-    op.apply(x, tmp);
+    C acc = rhs_norm2;
+    if constexpr (!ZERO_GUESS) {
+        op.apply(x, tmp);
 #pragma unroll
-    for (int i = 0; i < K; ++i) rhs[i] = rhs[i] - tmp[i];
-    C acc = op.wnorm2(rhs);
+        for (int i = 0; i < K; ++i) rhs[i] = rhs[i] - tmp[i];
+        acc = op.wnorm2(rhs);
+    }
     bool converged = acc <= tol2;
     int it = 0;
     for (int k = 0; k < Cfg::KRYLOV_MAX_ITERS; ++k) {
@@ -98,7 +101,7 @@ template <class R> __device__ __forceinline__ R clampd(R v, R lim) {
 // product to +-dot_clamp, flags BICGSTAB_BREAKDOWN when rho or omega
 // collapse (1e-30 in float32, 1e-200 in float64) or a recurrence quotient
 // would leave the clamp budget.
-template <class Cfg, class Op>
+template <class Cfg, class Op, bool ZERO_GUESS>
 __device__ __forceinline__ int solve_bicgstab(const Op& op, typename Cfg::R* rhs,
                                               typename Cfg::R* x, int& iters) {
     using R = typename Cfg::R;
@@ -119,12 +122,12 @@ __device__ __forceinline__ int solve_bicgstab(const Op& op, typename Cfg::R* rhs
     const C rhs_norm2 = op.wnorm2(rhs);
     const C tol = C(Cfg::KRYLOV_FLOOR) + C(Cfg::KRYLOV_REDUCTION) * sqrt_t(rhs_norm2);
     const C tol2 = tol * tol;
-    op.apply(x, tmp);
+    if constexpr (!ZERO_GUESS) op.apply(x, tmp);
     R rho_prev = R(0);
 #pragma unroll
     for (int i = 0; i < K; ++i) {
-        const R ax = clampd(tmp[i], lim);
-        const R ri = rhs[i] - ax;
+        R ri = rhs[i];
+        if constexpr (!ZERO_GUESS) ri = ri - clampd(tmp[i], lim);
         rhs[i] = ri;
         if constexpr (SHS) r0s[op.slot(i)] = ri;
         else r0[i] = ri;
@@ -134,7 +137,8 @@ __device__ __forceinline__ int solve_bicgstab(const Op& op, typename Cfg::R* rhs
         rho_prev += sq;
     }
     rho_prev = op.reduce(rho_prev);
-    C acc = op.wnorm2(rhs);
+    C acc = rhs_norm2;
+    if constexpr (!ZERO_GUESS) acc = op.wnorm2(rhs);
     bool converged = acc <= tol2;
     bool broken = false;
     bool finished = converged;
@@ -238,7 +242,7 @@ __device__ __forceinline__ int solve_bicgstab(const Op& op, typename Cfg::R* rhs
 // change the answer and only cost FP64 and conversion issue slots).  One
 // Arnoldi step (one operator and one preconditioner application) counts
 // as one iteration.
-template <class Cfg, class Op>
+template <class Cfg, class Op, bool ZERO_GUESS>
 __device__ __forceinline__ int solve_gmres(const Op& op, typename Cfg::R* rhs,
                                            typename Cfg::R* x, int& iters) {
     using R = typename Cfg::R;
@@ -267,14 +271,15 @@ __device__ __forceinline__ int solve_gmres(const Op& op, typename Cfg::R* rhs,
         return sqrt_t(op.reduce(s));
     };
 
-    const R tol = R(Cfg::KRYLOV_FLOOR) + R(Cfg::KRYLOV_REDUCTION) * scaled_norm(rhs);
-    op.apply(x, w);
+    R beta = scaled_norm(rhs);
+    const R tol = R(Cfg::KRYLOV_FLOOR) + R(Cfg::KRYLOV_REDUCTION) * beta;
+    if constexpr (!ZERO_GUESS) op.apply(x, w);
 #pragma unroll
     for (int i = 0; i < K; ++i) {
         b[i] = rhs[i];
-        rhs[i] = rhs[i] - w[i];
+        if constexpr (!ZERO_GUESS) rhs[i] = rhs[i] - w[i];
     }
-    R beta = scaled_norm(rhs);
+    if constexpr (!ZERO_GUESS) beta = scaled_norm(rhs);
     bool converged = beta <= tol;
     int it = 0;
     while (!converged && it < Cfg::KRYLOV_MAX_ITERS) {

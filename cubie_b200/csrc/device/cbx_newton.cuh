@@ -53,16 +53,19 @@ __device__ __forceinline__ typename Cfg::C weighted_norm2(const typename Cfg::R*
     return nrm2 * (C(1) / C(K));
 }
 
-template <class Cfg, class Op>
+// ``ZERO_GUESS``: x holds zeros on entry (every Newton correction), so the
+// first residual is the right-hand side itself and no operator is applied
+// for it.
+template <class Cfg, bool ZERO_GUESS = false, class Op>
 __device__ __forceinline__ int linear_solve(const Op& op, typename Cfg::R* rhs, typename Cfg::R* x, int& iters) {
     if constexpr (Cfg::LIN == LIN_BICGSTAB) {
-        return solve_bicgstab<Cfg, Op>(op, rhs, x, iters);
+        return solve_bicgstab<Cfg, Op, ZERO_GUESS>(op, rhs, x, iters);
     } else if constexpr (Cfg::LIN == LIN_GMRES) {
-        return solve_gmres<Cfg, Op>(op, rhs, x, iters);
+        return solve_gmres<Cfg, Op, ZERO_GUESS>(op, rhs, x, iters);
     } else if constexpr (Cfg::LIN == LIN_DIRECT) {
         return solve_direct<Cfg, Op>(op, rhs, x, iters);
     } else {
-        return solve_mr<Cfg, Op, Cfg::LIN == LIN_SD>(op, rhs, x, iters);
+        return solve_mr<Cfg, Op, Cfg::LIN == LIN_SD, ZERO_GUESS>(op, rhs, x, iters);
     }
 }
 
@@ -221,7 +224,7 @@ __device__ __forceinline__ int newton_solve(Prob& prob, typename Cfg::R* u, type
         }
         if constexpr (!HasFused<Prob>::value) prob.linearize(u);
         int kit = 0;
-        const int lin = linear_solve<Cfg>(prob.op(), res, delta, kit);
+        const int lin = linear_solve<Cfg, true>(prob.op(), res, delta, kit);
         total_k += kit;
         last_lin = lin;
         ++iters;

@@ -5,11 +5,13 @@
 // Layout: lane l of the warp holds components l, l + 32, l + 64, ... of
 // every state-sized vector (L = ceil(N / 32) values per lane, padded with
 // zeros).  The right-hand side and the Jacobian-vector product are
-// evaluated by the whole warp from copies in shared memory, through the
-// class-grouped generated functions (``WSys::dxdt_lanes`` /
-// ``WSys::jmv_lanes``; cubie_b200/warpgen.py).  Dot products and norms are
-// lane partials summed with shuffles and then broadcast from lane 0, so
-// every lane holds bit-identical scalars and all control flow (accept or
+// evaluated by the whole warp through generated functions
+// (cubie_b200/warpgen.py): per-lane code over registers and shuffles where
+// the system's couplings lie at constant offsets (``RegisterForm`` below),
+// otherwise class-grouped code over copies in shared memory
+// (``WSys::dxdt_lanes`` / ``WSys::jmv_lanes``).  Dot products and norms are
+// lane partials summed with a shuffle butterfly, which leaves the same bits
+// on every lane, so all control flow (accept or
 // reject, Newton and Krylov convergence, the event schedule) is uniform
 // across the warp.  The Krylov solvers and the Newton iteration are the
 // shared ones (cbx_linear.cuh, cbx_newton.cuh) instantiated on the warp
@@ -25,14 +27,36 @@ namespace cbx {
 
 constexpr unsigned kWarpFull = 0xffffffffu;
 
-// Sum over the warp, then lane 0's value everywhere (the butterfly alone
-// may round differently on different lanes).
+// Sum over the warp, the same bits on every lane: at each level the two
+// partners of a butterfly add the same two values, and addition commutes, so
+// no broadcast is needed after it.
 template <class T>
 __device__ __forceinline__ T warp_sum(T v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(kWarpFull, v, o);
-    return __shfl_sync(kWarpFull, v, 0);
+    return v;
 }
+
+// The register form of the system (cubie_b200/warpgen.py): every vector and
+// the Jacobian's coefficients stay in the lanes' registers, and J v takes one
+// shuffle per neighbour offset and a multiply-add per coefficient, where the
+// shared-memory form stores the operand, waits for the warp, reads operand,
+// coefficients and indices back and stores the result.  The generator offers
+// it when every read lies at a constant offset from the component it serves.
+// What bounds the kernel is the latency of those exchanges and the issue
+// slots of their loads and stores, not arithmetic or bandwidth.  Shared
+// against register form, Hodgkin-Huxley cables, l_stable_dirk_3 + BiCGSTAB,
+// 80 steps on one B200: 76 states x 5,003 runs 7.35 -> 3.33 ms, 256 x 1,536
+// 4.03 -> 1.44, 384 x 1,000 4.43 -> 1.56, 512 x 800 5.61 -> 2.27; FP64 256 x
+// 1,536 11.4 -> 8.6.  512 FP32 and 256 FP64 states (832 bytes a lane by the
+// count below) spill part of their vectors to local memory and still gain;
+// nothing larger was measured, so the rule ends there.
+template <class Cfg>
+struct RegisterForm {
+    static constexpr int L = (Cfg::N + 31) / 32;
+    static constexpr int BYTES = int(sizeof(typename Cfg::R)) * (10 * L + Cfg::WSys::NC);
+    static constexpr bool VALUE = Cfg::WSys::NC > 0 && BYTES <= 832;
+};
 
 // Per-warp shared memory.  With a cached Jacobian (WSys::NNZ > 0) the
 // linearisation stores J's nonzero coefficients in ``jac`` and every J v
@@ -45,13 +69,14 @@ template <class Cfg>
 struct WarpMem {
     using R = typename Cfg::R;
     static constexpr int N = Cfg::N;
+    static constexpr bool REG = RegisterForm<Cfg>::VALUE;
     static constexpr bool CACHED = Cfg::WSys::NNZ > 0;
     static constexpr int SH = Cfg::SHARED_SCRATCH ? N : 1;
-    R ys[N];                              // state of a right-hand-side evaluation
-    R vs[N];                              // operand of J v
-    R out[N];                             // class outputs
-    R kw[N];                              // Krylov weights 1 / tol_i of the current stage solve
-    R jac[CACHED ? Cfg::WSys::NNZ : 1];   // cached Jacobian coefficients
+    R ys[N];                              // state of a right-hand-side evaluation or of an output row
+    R vs[REG ? 1 : N];                    // operand of J v
+    R out[REG ? 1 : N];                   // class outputs
+    R kw[REG ? 1 : N];                    // Krylov weights 1 / tol_i of the current stage solve
+    R jac[CACHED && !REG ? Cfg::WSys::NNZ : 1];   // cached Jacobian coefficients
     R ylin[CACHED ? 1 : N];               // linearisation point (matrix-free J v)
     R sbase[SH];                          // stage base state (shared placement)
     R sstart[SH];                         // step start state (shared placement)
@@ -68,6 +93,9 @@ struct WarpCtx {
     using C = typename Cfg::C;
     static constexpr int N = Cfg::N, ND = Cfg::ND, L = (Cfg::N + 31) / 32;
     static constexpr bool CACHED = WarpMem<Cfg>::CACHED;
+    static constexpr bool REG = WarpMem<Cfg>::REG;
+    static constexpr int NC = REG ? Cfg::WSys::NC : 1;                     // register form: coefficients,
+    static constexpr int NG = REG && Cfg::WSys::NG > 0 ? Cfg::WSys::NG : 1;  // exchanged values per lane
     WarpMem<Cfg>* m;
     int lane;
     const R* coeffs;
@@ -91,22 +119,42 @@ struct WarpCtx {
         for (int q = 0; q < ND; ++q)
             if (lane == q) dst[q] = drv[q];
     }
+    // The values of ``loc`` that the lane's expressions read from other lanes
+    // (register form), in the generated plan's order.
+    __device__ __forceinline__ void gather(const R* loc, R* g) const {
+        if constexpr (REG) {
+#pragma unroll
+            for (int i = 0; i < Cfg::WSys::NG; ++i) {
+                const int k = Cfg::WSys::g_slot(i), s = Cfg::WSys::g_shift(i), mode = Cfg::WSys::g_mode(i);
+                const R first = (k >= 0 && k < L) ? loc[k >= 0 && k < L ? k : 0] : R(0);
+                const R second = (k + 1 >= 0 && k + 1 < L) ? loc[k + 1 >= 0 && k + 1 < L ? k + 1 : 0] : R(0);
+                const R src = mode == 1 ? first : (mode == 2 ? second : (lane >= s ? first : second));
+                g[i] = __shfl_sync(kWarpFull, src, (lane + s) & 31);
+            }
+        }
+    }
     // f(t, y): y and f local.  Every exchange is put -> sync -> class code
     // -> sync -> get: the second sync already orders every lane's reads of
     // the inputs before any later put, and every write of ``out`` comes after
     // the next exchange's first sync, so no sync follows the get.
     __device__ __forceinline__ void rhs(const R* yloc, R t, const R* drv, R* floc) const {
-        put(m->ys, yloc);
-        put_drivers(m->d, drv);
-        __syncwarp();
-        Cfg::WSys::template dxdt_lanes<R>(m->ys, m->p, m->d, t, m->out, lane);
-        __syncwarp();
-        get(m->out, floc);
+        if constexpr (REG) {
+            R g[NG];
+            gather(yloc, g);
+            Cfg::WSys::template f_reg<R>(yloc, g, m->p, drv, t, lane, floc);
+        } else {
+            put(m->ys, yloc);
+            put_drivers(m->d, drv);
+            __syncwarp();
+            Cfg::WSys::template dxdt_lanes<R>(m->ys, m->p, m->d, t, m->out, lane);
+            __syncwarp();
+            get(m->out, floc);
+        }
     }
-    __device__ __forceinline__ void linearize(const R* Yloc, R t, const R* drv) const {
+    __device__ __forceinline__ void linearize(const R* Yloc, R t, const R* drv, R* J) const {
         if constexpr (CACHED) {
             R scratch[L];
-            rhs_linearize(Yloc, t, drv, scratch);
+            rhs_linearize(Yloc, t, drv, scratch, J);
         } else {
             put(m->ylin, Yloc);
             put_drivers(m->dlin, drv);
@@ -116,9 +164,14 @@ struct WarpCtx {
     }
     // f(t, Y) and the linearisation at Y in one pass: with a cached
     // Jacobian, f and J's coefficients share their subexpressions (the
-    // exponentials of a gating rate appear in both).
-    __device__ __forceinline__ void rhs_linearize(const R* Yloc, R t, const R* drv, R* floc) const {
-        if constexpr (CACHED) {
+    // exponentials of a gating rate appear in both).  The register form
+    // leaves the lane's coefficients in ``J``.
+    __device__ __forceinline__ void rhs_linearize(const R* Yloc, R t, const R* drv, R* floc, R* J) const {
+        if constexpr (REG) {
+            R g[NG];
+            gather(Yloc, g);
+            Cfg::WSys::template fj_reg<R>(Yloc, g, m->p, drv, t, lane, floc, J);
+        } else if constexpr (CACHED) {
             put(m->ys, Yloc);
             put_drivers(m->d, drv);
             __syncwarp();
@@ -127,20 +180,27 @@ struct WarpCtx {
             get(m->out, floc);
         } else {
             rhs(Yloc, t, drv, floc);
-            linearize(Yloc, t, drv);
+            linearize(Yloc, t, drv, J);
         }
     }
-    // J(y_lin) v: v and the result local.
-    __device__ __forceinline__ void jmv(const R* vloc, R* outloc) const {
-        put(m->vs, vloc);
-        __syncwarp();
-        if constexpr (CACHED) {
-            Cfg::WSys::template jmv_cached<R>(m->vs, m->jac, m->out, lane);
+    // J(y_lin) v: v and the result local; ``J`` the register form's
+    // coefficients.
+    __device__ __forceinline__ void jmv(const R* vloc, const R* J, R* outloc) const {
+        if constexpr (REG) {
+            R g[NG];
+            gather(vloc, g);
+            Cfg::WSys::template jmv_reg<R>(vloc, g, J, outloc);
         } else {
-            Cfg::WSys::template jmv_lanes<R>(m->ylin, m->vs, m->p, m->dlin, tlin, m->out, lane);
+            put(m->vs, vloc);
+            __syncwarp();
+            if constexpr (CACHED) {
+                Cfg::WSys::template jmv_cached<R>(m->vs, m->jac, m->out, lane);
+            } else {
+                Cfg::WSys::template jmv_lanes<R>(m->ylin, m->vs, m->p, m->dlin, tlin, m->out, lane);
+            }
+            __syncwarp();
+            get(m->out, outloc);
         }
-        __syncwarp();
-        get(m->out, outloc);
     }
 };
 
@@ -155,11 +215,19 @@ struct WarpStageOp {
     static constexpr int K = WarpCtx<Cfg>::L;
     static constexpr int KT = Cfg::N;
     static constexpr bool SHADOW_SHARED = Cfg::SHARED_SCRATCH;
+    static constexpr bool REG = WarpCtx<Cfg>::REG;
+    static constexpr int KW = REG ? K : 1;
     WarpCtx<Cfg> w;   // by value: no address of the solve's state is taken
     R s;
+    R J[WarpCtx<Cfg>::NC];   // register form: the lane's coefficients and Krylov weights
+    R kwr[KW];
+    __device__ __forceinline__ R weight(int i) const {
+        if constexpr (REG) return kwr[i];
+        else return w.m->kw[w.lane + 32 * i];
+    }
     __device__ __forceinline__ void apply(const R* v, R* out) const {
         R jv[K];
-        w.jmv(v, jv);
+        w.jmv(v, J, jv);
 #pragma unroll
         for (int i = 0; i < K; ++i) out[i] = v[i] - s * jv[i];
     }
@@ -168,21 +236,20 @@ struct WarpStageOp {
         for (int i = 0; i < K; ++i) out[i] = v[i];
 #pragma unroll 1
         for (int k = 0; k < Cfg::PRECOND_ORDER; ++k) {
-            w.jmv(out, scratch);
+            w.jmv(out, J, scratch);
 #pragma unroll
             for (int i = 0; i < K; ++i) out[i] = v[i] + s * scratch[i];
         }
     }
     __device__ __forceinline__ C tol(int i) const {
-        const int c = w.lane + 32 * i;
-        return w.valid(i) ? C(R(1) / w.m->kw[c]) : C(1);
+        return w.valid(i) ? C(R(1) / weight(i)) : C(1);
     }
     __device__ __forceinline__ C wnorm2(const R* v) const {
         R s2 = R(0);
 #pragma unroll
         for (int i = 0; i < K; ++i) {
             if (w.valid(i)) {
-                const R ratio = v[i] * w.m->kw[w.lane + 32 * i];
+                const R ratio = v[i] * weight(i);
                 s2 += ratio * ratio;
             }
         }
@@ -237,6 +304,8 @@ struct WarpDirkProblem {
     R start_v[KL];
     R drv[ND > 0 ? ND : 1];
     R t, h, a;
+    R J[WarpCtx<Cfg>::NC];                       // register form: coefficients at the last linearisation
+    R kwr[WarpStageOp<Cfg>::KW];                 // and the stage solve's Krylov weights
     __device__ __forceinline__ R b(int k) const {
         if constexpr (Cfg::SHARED_SCRATCH) return w.valid(k) ? w.m->sbase[w.lane + 32 * k] : R(0);
         else if constexpr (Cfg::REG_SCRATCH) return base_v[k];
@@ -259,7 +328,7 @@ struct WarpDirkProblem {
         R Y[K];
 #pragma unroll
         for (int k = 0; k < K; ++k) Y[k] = b(k) + a * z[k];
-        w.linearize(Y, t, drv);
+        w.linearize(Y, t, drv, J);
     }
     // residual and linearisation at the same iterate (the Newton loop
     // evaluates both at every iteration)
@@ -267,25 +336,37 @@ struct WarpDirkProblem {
         R Y[K], f[K];
 #pragma unroll
         for (int k = 0; k < K; ++k) Y[k] = b(k) + a * z[k];
-        w.rhs_linearize(Y, t, drv, f);
+        w.rhs_linearize(Y, t, drv, f, J);
 #pragma unroll
         for (int k = 0; k < K; ++k) out[k] = w.valid(k) ? z[k] - h * f[k] : R(0);
     }
-    __device__ __forceinline__ WarpStageOp<Cfg> op() const { return WarpStageOp<Cfg>{w, a * h}; }
+    __device__ __forceinline__ WarpStageOp<Cfg> op() const {
+        WarpStageOp<Cfg> o{w, a * h, {}, {}};
+        if constexpr (WarpCtx<Cfg>::REG) {
+#pragma unroll
+            for (int i = 0; i < WarpCtx<Cfg>::NC; ++i) o.J[i] = J[i];
+#pragma unroll
+            for (int k = 0; k < K; ++k) o.kwr[k] = kwr[k];
+        }
+        return o;
+    }
     // Krylov weights 1 / max(katol + krtol * scale * |base|, 1e-16), once per
     // stage solve
-    __device__ __forceinline__ void form_weights() const {
+    __device__ __forceinline__ void form_weights() {
 #pragma unroll
         for (int k = 0; k < K; ++k) {
+            if constexpr (WarpCtx<Cfg>::REG) kwr[k] = R(0);
             if (!w.valid(k)) continue;
             const int c = w.lane + 32 * k;
+            R v;
             if constexpr (Cfg::MIXED)
-                w.m->kw[c] = R(1) / pymax(R(Cfg::katol(c)) + R(Cfg::krtol(c)) * R(w.tol_scale) * absv(b(k)),
-                                          R(1e-16));
+                v = R(1) / pymax(R(Cfg::katol(c)) + R(Cfg::krtol(c)) * R(w.tol_scale) * absv(b(k)), R(1e-16));
             else
-                w.m->kw[c] = R(C(1) / krylov_tol<Cfg>(c, b(k), w.tol_scale));
+                v = R(C(1) / krylov_tol<Cfg>(c, b(k), w.tol_scale));
+            if constexpr (WarpCtx<Cfg>::REG) kwr[k] = v;
+            else w.m->kw[c] = v;
         }
-        __syncwarp();
+        if constexpr (!WarpCtx<Cfg>::REG) __syncwarp();
     }
     __device__ __forceinline__ C corr_norm2(const R* delta, const R* z) const {
         C nrm2 = C(0);
@@ -340,7 +421,7 @@ struct WarpDirkStep {
     // them, more live registers around the call).  The autotuner picks.
     static __device__ CBX_NOINLINE int stage_solve(WarpCtx<Cfg> w, const R* base, const R* y, const R* drv_stage,
                                                       R stage_time, R dt, R a, R* z_io, C& theta, int2& iters) {
-        WarpDirkProblem<Cfg> prob{w, base, y, {}, {}, {}, stage_time, dt, a};
+        WarpDirkProblem<Cfg> prob{w, base, y, {}, {}, {}, stage_time, dt, a, {}, {}};
 #pragma unroll
         for (int q = 0; q < ND; ++q) prob.drv[q] = drv_stage[q];
         prob.form_weights();
@@ -364,7 +445,7 @@ struct WarpDirkStep {
     }
     static __device__ CBX_NOINLINE WarpStageOut<Cfg> stage_solve_regs(WarpCtx<Cfg> w, WarpStageIn<Cfg> in,
                                                                        R stage_time, R dt, R a, C theta) {
-        WarpDirkProblem<Cfg> prob{w, nullptr, nullptr, {}, {}, {}, stage_time, dt, a};
+        WarpDirkProblem<Cfg> prob{w, nullptr, nullptr, {}, {}, {}, stage_time, dt, a, {}, {}};
 #pragma unroll
         for (int k = 0; k < L; ++k) {
             prob.base_v[k] = in.base[k];

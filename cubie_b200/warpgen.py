@@ -249,6 +249,194 @@ def _emit_cached_jacobian(classes: List[ExprClass], tables: List[str]):
     return "\n".join(fj), "\n".join(jm), base, fl_fj, fl_jm
 
 
+# Largest register form the generator emits (see ``_register_plan``).  The
+# device code decides by its working precision whether the lanes can hold it.
+REGISTER_MAX_SLOTS = 16      # vector components per lane (512 states)
+REGISTER_MAX_COEFS = 64      # Jacobian coefficients per lane
+REGISTER_MAX_GATHERS = 40    # exchanged values per J v
+
+
+@dataclass
+class RegisterBody:
+    """One class evaluated for one slot: lane ``l`` of ``lanes`` evaluates
+    component ``l + 32 slot``."""
+
+    cls: int
+    slot: int
+    lanes: List[int]
+    offsets: List[object]        # per placeholder: int offset (y, v), index expression text (p, d)
+
+
+@dataclass
+class RegisterPlan:
+    bodies_f: List[RegisterBody]                      # f alone
+    bodies_fj: List[RegisterBody]                     # f and the Jacobian's coefficients
+    gathers: List[Tuple[int, int, int]]               # (slot, shift, mode) of every exchanged value
+    gather_of: Dict[Tuple[int, int], int]             # (slot, offset) -> exchange, absent when the lane holds it
+    coefs: Dict[Tuple[int, int], int]                 # (slot, offset) -> coefficient
+
+
+def _register_bodies(classes: List[ExprClass]) -> List[RegisterBody]:
+    bodies: Dict[tuple, RegisterBody] = {}
+    for ci, c in enumerate(classes):
+        for row, comp in zip(c.indices, c.members):
+            offs: List[object] = [idx - comp if kind in "yv" else idx for (kind, _), idx in zip(c.slots, row)]
+            b = bodies.setdefault((comp // 32, ci, tuple(offs)), RegisterBody(ci, comp // 32, [], offs))
+            b.lanes.append(comp % 32)
+    return [bodies[k] for k in sorted(bodies, key=lambda k: (k[0], bodies[k].lanes[0], k[1]))]
+
+
+def _merged_order(sequences: List[List[int]]) -> List[int]:
+    """The distinct items of ``sequences`` in an order that keeps every
+    sequence's own (first-seen order where they contradict each other)."""
+    items = list(dict.fromkeys(d for seq in sequences for d in seq))
+    before: Dict[int, set] = {d: set() for d in items}
+    for seq in sequences:
+        for a, b in zip(seq, seq[1:]):
+            before[b].add(a)
+    out: List[int] = []
+    while len(out) < len(items):
+        left = [d for d in items if d not in out]
+        out.append(next((d for d in left if before[d] <= set(out)), left[0]))
+    return out
+
+
+def _register_plan(n: int, classes_f: List[ExprClass], classes_fj: List[ExprClass]):
+    """How a warp evaluates ``classes_f`` (of f_i) and ``classes_fj`` (of the
+    joint expression (f_i, (J v)_i)) with every vector spread over its lanes'
+    registers, or None when it cannot.
+
+    Lane ``l`` holds components ``l + 32 k`` in slot ``k``.  When the
+    component an expression reads lies at a constant offset ``d`` from the
+    component it computes (neighbours on a line, the same compartment's other
+    variables), the read is a rotation of the vector by ``d``: with
+    ``d = 32 q + s`` lane ``l`` needs slot ``k + q`` (or ``k + q + 1`` past the
+    end of the warp) of lane ``(l + s) % 32``.  Every source lane serves
+    exactly one lane, so it first selects the slot it is asked for and one
+    shuffle moves it; ``s = 0`` needs neither.  Members of a class that read
+    at different offsets become separate bodies.
+
+    A gather's mode: 0 selects between the two slots, 1 only the first is
+    ever read, 2 only the second."""
+    slots = (n + 31) // 32
+    bodies_f, bodies_fj = _register_bodies(classes_f), _register_bodies(classes_fj)
+    if slots > REGISTER_MAX_SLOTS or max(len(bodies_f), len(bodies_fj)) > 3 * slots + 4:
+        return None
+    need: Dict[Tuple[int, int], set] = {}             # (slot + q, s) -> {False: first slot read, True: second}
+    gather_keys: Dict[Tuple[int, int], Tuple[int, int]] = {}
+    coefs: Dict[Tuple[int, int], int] = {}
+    for classes, bodies in ((classes_f, bodies_f), (classes_fj, bodies_fj)):
+        for b in bodies:
+            for (kind, _), d in zip(classes[b.cls].slots, b.offsets):
+                if kind not in "yv":
+                    continue
+                q, s = divmod(d, 32)
+                if s:
+                    gather_keys[(b.slot, d)] = (b.slot + q, s)
+                    need.setdefault((b.slot + q, s), set()).update(l + s >= 32 for l in b.lanes)
+    # each row sums its terms in its own class's order (zero coefficients of
+    # the slot's other classes in between), so a J v rounds as the
+    # shared-memory form's does
+    for k in range(slots):
+        rows = [[d for (kind, _), d in zip(classes_fj[b.cls].slots, b.offsets) if kind == "v"]
+                for b in bodies_fj if b.slot == k]
+        for d in _merged_order(rows):
+            coefs[(k, d)] = len(coefs)
+    if len(coefs) > REGISTER_MAX_COEFS or len(need) > REGISTER_MAX_GATHERS:
+        return None
+    order = sorted(need)
+    gathers = [(k, s, 0 if len(need[(k, s)]) == 2 else (2 if True in need[(k, s)] else 1)) for k, s in order]
+    gather_of = {key: order.index(ks) for key, ks in gather_keys.items()}
+    return RegisterPlan(bodies_f, bodies_fj, gathers, gather_of, coefs)
+
+
+def _lane_condition(lanes: List[int], n: int, slot: int) -> str:
+    """Condition on ``lane`` for ``lanes`` of a slot ("" when every lane)."""
+    if len(lanes) == 32:
+        return ""
+    lo, hi = min(lanes), max(lanes)
+    if len(lanes) == hi - lo + 1:
+        if lo == hi:
+            return f"lane == {lo}"
+        if lo == 0:
+            return f"lane < {hi + 1}"
+        return f"lane >= {lo}" if hi == 31 else f"(lane >= {lo} && lane < {hi + 1})"
+    return f"((0x{sum(1 << l for l in lanes):x}u >> lane) & 1u)"
+
+
+def _emit_register_lanes(n: int, classes_f: List[ExprClass], classes_fj: List[ExprClass],
+                         plan: RegisterPlan) -> str:
+    """The per-lane functions of the register form.  ``y`` / ``v`` are the
+    lane's slots, ``g`` the exchanged values in the plan's order, ``J`` the
+    lane's Jacobian coefficients (zero where a lane's row has none)."""
+    slots = (n + 31) // 32
+
+    def read(vec: str, slot: int, d: int) -> str:
+        q, s = divmod(d, 32)
+        return f"{vec}[{slot + q}]" if s == 0 else f"g[{plan.gather_of[(slot, d)]}]"
+
+    def body_lines(b: RegisterBody, with_j: bool) -> List[str]:
+        c = (classes_fj if with_j else classes_f)[b.cls]
+        f_t, jv_t = c.template.args if with_j else (c.template, sp.Integer(0))
+        sym_map = {TIME: "t"}
+        lines = []
+        v_syms = []
+        for (kind, j), d in zip(c.slots, b.offsets):
+            ph = _placeholder(kind, j)
+            if kind == "v":
+                v_syms.append((ph, d))
+                continue
+            sym_map[ph] = (read("y", b.slot, d) if kind == "y" else f"{'ps' if kind == 'p' else 'ds'}[{d}]")
+        coefs = [sp.diff(jv_t, v) for v, _ in v_syms]
+        if any(v in cf.free_symbols for cf in coefs for v, _ in v_syms):
+            raise ValueError("Jacobian-vector template is not linear in v")
+        printer = _CudaPrinter(sym_map)
+        reps, reduced = sp.cse([f_t, *coefs], symbols=sp.numbered_symbols("_t"), optimizations="basic")
+        for sy, e in reps:
+            lines.append(f"const R {sy} = {printer.doprint(e)};")
+        lines.append(f"f[{b.slot}] = {printer.doprint(reduced[0])};")
+        for (_, d), e in zip(v_syms, reduced[1:]):
+            lines.append(f"J[{plan.coefs[(b.slot, d)]}] = {printer.doprint(e)};")
+        return lines
+
+    def evaluate(name: str, with_j: bool) -> List[str]:
+        out = [f"    template <class R> static __device__ __forceinline__ void {name}(const R* y, const R* g, "
+               f"const R* __restrict__ ps, const R* ds, R t, int lane, R* f{', R* J' if with_j else ''})", "    {",
+               "        (void)y; (void)g; (void)ps; (void)ds; (void)t; (void)lane;"]
+        bodies = plan.bodies_fj if with_j else plan.bodies_f
+        covered: Dict[int, int] = {}
+        for b in bodies:
+            covered[b.slot] = max(covered.get(b.slot, 0), len(b.lanes))
+        for k in range(slots):
+            if covered.get(k, 0) < 32:
+                out.append(f"        f[{k}] = R(0);")
+        if with_j:
+            for (k, _), i in plan.coefs.items():
+                if covered.get(k, 0) < 32:
+                    out.append(f"        J[{i}] = R(0);")
+        for b in bodies:
+            cond = _lane_condition(b.lanes, n, b.slot)
+            out.append(f"        {'if (' + cond + ') ' if cond else ''}{{")
+            out += ["            " + ln for ln in body_lines(b, with_j)]
+            out.append("        }")
+        return out + ["    }"]
+
+    jm = ["    template <class R> static __device__ __forceinline__ void jmv_reg(const R* v, const R* g, const R* J, "
+          "R* out)", "    {", "        (void)v; (void)g; (void)J;"]
+    for k in range(slots):
+        terms = [f"J[{i}] * {read('v', kk, d)}" for (kk, d), i in plan.coefs.items() if kk == k]
+        jm.append(f"        out[{k}] = {' + '.join(terms) if terms else 'R(0)'};")
+    jm.append("    }")
+    tables = []
+    for q, fn in enumerate(("g_slot", "g_shift", "g_mode")):
+        vals = [str(g[q]) for g in plan.gathers] or ["0"]
+        tables.append(f"    static __device__ constexpr int {fn}(int i) {{ constexpr int v[{len(vals)}] = "
+                      f"{{{', '.join(vals)}}}; return v[i]; }}")
+    return "\n".join([f"    static constexpr int NC = {len(plan.coefs)};   // coefficients per lane",
+                      f"    static constexpr int NG = {len(plan.gathers)};   // exchanged values per lane",
+                      *tables, *evaluate("f_reg", False), *evaluate("fj_reg", True), *jm])
+
+
 def generate_warp_system(system: SymbolicODE, struct_name: str = "WarpSystem") -> WarpSystemCode:
     """Class-grouped right-hand side and Jacobian-vector product."""
     n = system.num_states
@@ -280,10 +468,14 @@ def generate_warp_system(system: SymbolicODE, struct_name: str = "WarpSystem") -
     # together with f, then every J v is a short sum over shared memory
     nnz = sum(1 for i in range(n) for k in range(n) if J[i, k] != 0)
     cached, n_fj = [], 0
+    register = "    static constexpr int NC = 0, NG = 0;"
     if 0 < nnz <= CACHED_JAC_MAX:
         cfj = group_classes([sp.Tuple(f[i], jv[i]) for i in range(n)], kind_v)
         body_fj, body_jc, stored, fl_fj, fl_jc = _emit_cached_jacobian(cfj, tables)
         cached = [body_fj, body_jc]
+        plan = _register_plan(n, cf, cfj)
+        if plan is not None:
+            register = _emit_register_lanes(n, cf, cfj, plan)
         n_fj = len(cfj)
         nnz = stored
         flops.update({"fj": fl_fj, "jmv_cached": fl_jc})
@@ -295,6 +487,7 @@ def generate_warp_system(system: SymbolicODE, struct_name: str = "WarpSystem") -
            f"    static constexpr int NP = {system.num_parameters};",
            f"    static constexpr int ND = {system.num_drivers};",
            f"    static constexpr int NNZ = {nnz};",
+           register,
            body_f,
            body_j,
            *cached,
