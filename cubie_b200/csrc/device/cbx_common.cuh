@@ -41,9 +41,36 @@ enum Ctrl : int { CTRL_FIXED = 0, CTRL_I = 1, CTRL_PI = 2, CTRL_PID = 3, CTRL_GU
 // strictly larger/smaller; this decides NaN propagation).
 template <class T> __device__ __forceinline__ T pymax(T a, T b) { return (b > a) ? b : a; }
 template <class T> __device__ __forceinline__ T pymin(T a, T b) { return (b < a) ? b : a; }
-template <class T> __device__ __forceinline__ T clampv(T v, T lo, T hi) { return pymax(lo, pymin(v, hi)); }
 
-template <class T> __device__ __forceinline__ T absv(T v) { return v < T(0) ? -v : v; }
+// |v| (a free operand modifier on the device).
+__device__ __forceinline__ float absv(float v) { return fabsf(v); }
+__device__ __forceinline__ double absv(double v) { return fabs(v); }
+
+// max and min in one instruction, NaN when either operand is one.  They equal
+// pymax / pymin wherever a NaN can only come first (or comes in both), which
+// is a compare and a select otherwise.
+template <class T> __device__ __forceinline__ T max_nan(T a, T b) { return (b > a) ? b : a; }
+template <class T> __device__ __forceinline__ T min_nan(T a, T b) { return (b < a) ? b : a; }
+#ifndef CBX_HOST_EMULATION
+template <> __device__ __forceinline__ float max_nan<float>(float a, float b) {
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+template <> __device__ __forceinline__ float min_nan<float>(float a, float b) {
+    float r;
+    asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+#endif
+
+// v clamped to [lo, hi]; lo for a NaN.
+template <class T> __device__ __forceinline__ T clampv(T v, T lo, T hi) { return pymax(lo, pymin(v, hi)); }
+#ifndef CBX_HOST_EMULATION
+template <> __device__ __forceinline__ float clampv<float>(float v, float lo, float hi) {
+    return fmaxf(lo, min_nan(v, hi));   // fmaxf drops the NaN
+}
+#endif
 
 // A round-to-nearest add the compiler never fuses with the multiply that
 // produced an operand.  Used where a value crosses from the step function

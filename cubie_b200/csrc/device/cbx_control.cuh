@@ -54,8 +54,8 @@ struct Controller {
     static __device__ __forceinline__ G gpow(G a, G b) { return pow_t(a, b); }
     // One component's ratio max(|e|, 1e-16) / (atol + rtol s max(|y_new|, |y|)).
     static __device__ __forceinline__ G error_ratio(R e_i, R ynew_i, R y_i, G atol, G rtol, G ts) {
-        const G e = pymax(G(absv(e_i)), G(1e-16));
-        const G tol = atol + rtol * ts * pymax(G(absv(ynew_i)), G(absv(y_i)));
+        const G e = max_nan(G(absv(e_i)), G(1e-16));
+        const G tol = atol + rtol * ts * max_nan(G(absv(ynew_i)), G(absv(y_i)));
         return e / tol;
     }
     static __device__ __forceinline__ C error_norm2(const R* ynew, const R* y, const R* err, G ts) {
@@ -74,7 +74,7 @@ struct Controller {
             const bool within = (gain >= G(Cfg::CTL_DEADBAND_MIN)) && (gain <= G(Cfg::CTL_DEADBAND_MAX));
             gain = within ? G(1) : gain;
         }
-        return accept ? gain : pymin(gain, G(Cfg::CTL_SAFETY));
+        return accept ? gain : min_nan(gain, G(Cfg::CTL_SAFETY));
     }
     // Returns the controller status bits; updates dt, accept and history.
     // ``ts``: the run's tolerance scale in the gain precision

@@ -92,8 +92,7 @@ template <class Op> struct ShadowShared<Op, decltype(void(Op::SHADOW_SHARED))> {
 };
 
 template <class R> __device__ __forceinline__ R clampd(R v, R lim) {
-    v = (v > lim) ? lim : v;
-    return (v < -lim) ? -lim : v;
+    return max_nan(min_nan(v, lim), -lim);
 }
 
 // Preconditioned BiCGSTAB with the reference's breakdown and overflow
@@ -133,7 +132,7 @@ __device__ __forceinline__ int solve_bicgstab(const Op& op, typename Cfg::R* rhs
         else r0[i] = ri;
         p[i] = clampd(ri, lim);
         R sq = ri * ri;
-        sq = (sq > lim) ? lim : sq;
+        sq = min_nan(sq, lim);
         rho_prev += sq;
     }
     rho_prev = op.reduce(rho_prev);
@@ -190,7 +189,7 @@ __device__ __forceinline__ int solve_bicgstab(const Op& op, typename Cfg::R* rhs
             tmp[i] = clampd(tmp[i], lim);
             dot_ts += clampd(tmp[i] * rhs[i], lim);
             R sq = tmp[i] * tmp[i];
-            dot_tt += (sq > lim) ? lim : sq;
+            dot_tt += min_nan(sq, lim);
         }
         dot_ts = op.reduce(dot_ts);
         dot_tt = op.reduce(dot_tt);

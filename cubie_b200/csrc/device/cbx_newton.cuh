@@ -14,7 +14,7 @@ __device__ __forceinline__ typename Cfg::C krylov_tol(int i, typename Cfg::R ref
     using C = typename Cfg::C;
     const int k = i % Cfg::N;
     C t = C(Cfg::katol(k)) + C(Cfg::krtol(k)) * scale * C(absv(ref));
-    return pymax(t, C(1e-16));
+    return max_nan(t, C(1e-16));
 }
 
 // One component's ratio v / max(atol + rtol scale |ref|, 1e-16) of a
@@ -30,11 +30,11 @@ __device__ __forceinline__ typename Cfg::C tol_ratio(typename Cfg::R v, typename
     using R = typename Cfg::R;
     using C = typename Cfg::C;
     if constexpr (Cfg::MIXED) {
-        const R tol = pymax(R(atol) + R(rtol) * R(scale) * absv(ref), R(1e-16));
+        const R tol = max_nan(R(atol) + R(rtol) * R(scale) * absv(ref), R(1e-16));
         return C(v / tol);
     } else {
         C tol = C(atol) + C(rtol) * scale * C(absv(ref));
-        tol = pymax(tol, C(1e-16));
+        tol = max_nan(tol, C(1e-16));
         return C(v) / tol;
     }
 }

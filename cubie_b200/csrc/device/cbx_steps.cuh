@@ -450,7 +450,7 @@ struct FirkProblem {
             stage_state(u, i, Y);
 #pragma unroll
             for (int k = 0; k < N; ++k) {
-                const R ref = pymax(absv(Y[k]), absv(base[k]));
+                const R ref = max_nan(absv(Y[k]), absv(base[k]));
                 const C ratio = tol_ratio<Cfg>(delta[i * N + k], ref, Cfg::natol(k), Cfg::nrtol(k), ctx->tol_scale);
                 nrm2 += ratio * ratio;
             }
@@ -636,7 +636,7 @@ struct DirkProblem {
 #pragma unroll
         for (int k = 0; k < N; ++k) {
             const R sv = base[k] + a * z[k];
-            const R ref = pymax(absv(sv), absv(step_start[k]));
+            const R ref = max_nan(absv(sv), absv(step_start[k]));
             const C ratio = tol_ratio<Cfg>(delta[k], ref, Cfg::natol(k), Cfg::nrtol(k), ctx->tol_scale);
             nrm2 += ratio * ratio;
         }

@@ -360,7 +360,7 @@ struct WarpDirkProblem {
             const int c = w.lane + 32 * k;
             R v;
             if constexpr (Cfg::MIXED)
-                v = R(1) / pymax(R(Cfg::katol(c)) + R(Cfg::krtol(c)) * R(w.tol_scale) * absv(b(k)), R(1e-16));
+                v = R(1) / max_nan(R(Cfg::katol(c)) + R(Cfg::krtol(c)) * R(w.tol_scale) * absv(b(k)), R(1e-16));
             else
                 v = R(C(1) / krylov_tol<Cfg>(c, b(k), w.tol_scale));
             if constexpr (WarpCtx<Cfg>::REG) kwr[k] = v;
@@ -375,7 +375,7 @@ struct WarpDirkProblem {
             if (!w.valid(k)) continue;
             const int c = w.lane + 32 * k;
             const R sv = b(k) + a * z[k];
-            const R ref = pymax(absv(sv), absv(y0(k)));
+            const R ref = max_nan(absv(sv), absv(y0(k)));
             const C ratio = tol_ratio<Cfg>(delta[k], ref, Cfg::natol(c), Cfg::nrtol(c), w.tol_scale);
             nrm2 += ratio * ratio;
         }
