@@ -97,6 +97,7 @@ EXPORTED = (
     "cbx_module_load", "cbx_module_create", "cbx_module_destroy", "cbx_kernel_info",
     "cbx_occupancy", "cbx_solve", "cbx_device_info", "cbx_fp32_peak_probe", "cbx_flush_l2",
     "cbx_solve_noalloc", "cbx_adjoint_info", "cbx_adjoint_tape_bytes", "cbx_adjoint_launch", "cbx_solve_hetero",
+    "cbx_claim_order",
 )
 
 _lib = None
@@ -149,6 +150,8 @@ def lib():
         L.cbx_fp32_peak_probe.argtypes = [ctypes.c_int, ctypes.POINTER(ctypes.c_double),
                                           ctypes.POINTER(ctypes.c_float)]
         L.cbx_flush_l2.argtypes = [ctypes.c_void_p, ctypes.c_size_t, ctypes.c_void_p]
+        L.cbx_claim_order.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_double, ctypes.c_longlong,
+                                      ctypes.c_void_p, ctypes.c_void_p, ctypes.c_size_t, ctypes.c_void_p]
         L.cbx_solve_noalloc.argtypes = [ctypes.c_void_p, ctypes.POINTER(SolveArgs), ctypes.c_int, ctypes.c_int,
                                         ctypes.c_void_p]
         L.cbx_solve_hetero.argtypes = [ctypes.c_void_p, ctypes.POINTER(HeteroArgs), ctypes.c_int, ctypes.c_int,
@@ -294,6 +297,16 @@ def fp32_peak(device: int = 0) -> float:
     fl, ms = ctypes.c_double(), ctypes.c_float()
     _check(lib().cbx_fp32_peak_probe(device, ctypes.byref(fl), ctypes.byref(ms)), "cbx_fp32_peak_probe")
     return fl.value / (ms.value * 1e-3)
+
+
+CLAIM_ORDER_SCRATCH_BYTES = 16384
+
+
+def claim_order(work_ptr: int, scale_ptr: Optional[int], exponent: float, n: int, order_ptr: int, scratch_ptr: int,
+                stream: int = 0) -> None:
+    _check(lib().cbx_claim_order(ctypes.c_void_p(work_ptr), ctypes.c_void_p(scale_ptr), exponent, n,
+                                 ctypes.c_void_p(order_ptr), ctypes.c_void_p(scratch_ptr), CLAIM_ORDER_SCRATCH_BYTES,
+                                 ctypes.c_void_p(stream)), "cbx_claim_order")
 
 
 def flush_l2(buffer_ptr: int, nbytes: int, stream: int = 0) -> None:

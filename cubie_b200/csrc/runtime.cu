@@ -587,6 +587,136 @@ __global__ void __launch_bounds__(256) fp32_probe_kernel(float* out, float a, fl
     if (s == 1.2345f) out[blockIdx.x * blockDim.x + threadIdx.x] = s;
 }
 
+// ---------------------------------------------------------------------------
+// Claim order of a persistent launch: runs by decreasing estimated work.
+//
+// The order decides only when a run is claimed, so runs within a few percent
+// of each other need no order between them: a counting sort over bins of
+// log2(work), sixteen to an octave, takes the place of a full sort (a radix
+// sort of the 64-bit keys was twenty launches: 86 us of GPU time at 20,011
+// runs, 165 us at 2^20).  What bounds it is launches, not the 16 bytes it
+// moves per run: one block does all of it in shared memory for small batches;
+// at 20,011 runs one SM's load latency shows (18 us), where a counting and a
+// scattering launch over tiles take 9.5 us (65,536 runs; 15 us at 2^20), so
+// the line is drawn at one tile.
+// ---------------------------------------------------------------------------
+constexpr int kOrderBins = 2048;
+constexpr int kOrderThreads = 1024;
+constexpr int kOrderTile = 4096;
+constexpr long long kOrderOneBlock = kOrderTile;
+
+// Bin 0 holds the longest runs.  Anything log2 cannot place (a zero or
+// negative horizon, a NaN) lands in an end bin.
+__device__ __forceinline__ int order_bin(const double* work, const double* scale, float exponent, long long i) {
+    // rounded the same in every kernel: the counts must match the scatter
+    float l = log2f((float)work[i]);
+    if (scale) l = __fmaf_rn(exponent, log2f((float)scale[i]), l);
+    const float b = __fmul_rn(__fsub_rn(64.f, l), 16.f);
+    return int(fminf(fmaxf(b, 0.f), float(kOrderBins - 1)));   // a NaN: bin 0
+}
+
+// Exclusive prefix sums of the block's kOrderBins counts, in place.
+__device__ __forceinline__ void order_scan(unsigned* bins, unsigned* warp_sums) {
+    constexpr int per = kOrderBins / kOrderThreads;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    unsigned v[per], sum = 0;
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < per; ++k) {
+        v[k] = bins[t * per + k];
+        sum += v[k];
+    }
+    unsigned incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned up = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += up;
+    }
+    if (lane == 31) warp_sums[warp] = incl;
+    __syncthreads();
+    if (warp == 0) {
+        unsigned w = warp_sums[lane];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned up = __shfl_up_sync(0xffffffffu, w, o);
+            if (lane >= o) w += up;
+        }
+        warp_sums[lane] = w;
+    }
+    __syncthreads();
+    unsigned base = incl - sum + (warp ? warp_sums[warp - 1] : 0u);
+#pragma unroll
+    for (int k = 0; k < per; ++k) {
+        bins[t * per + k] = base;
+        base += v[k];
+    }
+    __syncthreads();
+}
+
+__global__ void __launch_bounds__(kOrderThreads) order_one_block_kernel(const double* work, const double* scale,
+                                                                        float exponent, int n, long long* order) {
+    __shared__ unsigned bins[kOrderBins];
+    __shared__ unsigned warp_sums[32];
+    for (int k = threadIdx.x; k < kOrderBins; k += kOrderThreads) bins[k] = 0u;
+    __syncthreads();
+#pragma unroll 4
+    for (int i = threadIdx.x; i < n; i += kOrderThreads) atomicAdd(bins + order_bin(work, scale, exponent, i), 1u);
+    order_scan(bins, warp_sums);
+#pragma unroll 4
+    for (int i = threadIdx.x; i < n; i += kOrderThreads)
+        order[atomicAdd(bins + order_bin(work, scale, exponent, i), 1u)] = i;
+}
+
+// counts: kOrderBins zeroed words
+__global__ void __launch_bounds__(kOrderThreads) order_count_kernel(const double* work, const double* scale,
+                                                                    float exponent, long long n, unsigned* counts) {
+    __shared__ unsigned bins[kOrderBins];
+    for (int k = threadIdx.x; k < kOrderBins; k += kOrderThreads) bins[k] = 0u;
+    __syncthreads();
+    const long long first = (long long)blockIdx.x * kOrderTile;
+    const long long last = first + kOrderTile < n ? first + kOrderTile : n;
+    for (long long i = first + threadIdx.x; i < last; i += kOrderThreads)
+        atomicAdd(bins + order_bin(work, scale, exponent, i), 1u);
+    __syncthreads();
+    for (int k = threadIdx.x; k < kOrderBins; k += kOrderThreads)
+        if (bins[k]) atomicAdd(counts + k, bins[k]);
+}
+
+// Each tile reserves a range of every bin it holds runs of, then fills it.
+// taken: kOrderBins zeroed words, the entries of each bin handed out so far.
+__global__ void __launch_bounds__(kOrderThreads) order_scatter_kernel(const double* work, const double* scale,
+                                                                      float exponent, long long n,
+                                                                      const unsigned* counts, unsigned* taken,
+                                                                      long long* order) {
+    __shared__ unsigned start[kOrderBins];
+    __shared__ unsigned bins[kOrderBins];
+    __shared__ unsigned warp_sums[32];
+    for (int k = threadIdx.x; k < kOrderBins; k += kOrderThreads) {
+        start[k] = counts[k];
+        bins[k] = 0u;
+    }
+    order_scan(start, warp_sums);
+    const long long first = (long long)blockIdx.x * kOrderTile;
+    int bin[kOrderTile / kOrderThreads];
+    unsigned at[kOrderTile / kOrderThreads];
+#pragma unroll
+    for (int q = 0; q < kOrderTile / kOrderThreads; ++q) {
+        const long long i = first + threadIdx.x + (long long)q * kOrderThreads;
+        bin[q] = -1;
+        if (i < n) {
+            bin[q] = order_bin(work, scale, exponent, i);
+            at[q] = atomicAdd(bins + bin[q], 1u);
+        }
+    }
+    __syncthreads();
+    for (int k = threadIdx.x; k < kOrderBins; k += kOrderThreads)
+        if (bins[k]) start[k] += atomicAdd(taken + k, bins[k]);
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < kOrderTile / kOrderThreads; ++q)
+        if (bin[q] >= 0) order[start[bin[q]] + at[q]] = first + threadIdx.x + (long long)q * kOrderThreads;
+}
+
 __global__ void flush_kernel(uint4* buf, size_t n16) {
     size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
     size_t stride = (size_t)gridDim.x * blockDim.x;
@@ -620,6 +750,32 @@ extern "C" int cbx_fp32_peak_probe(int device, double* flops, float* millisecond
     if (err != cudaSuccess) return fail(CBX_ERR_RUNTIME, "probe failed: %s", cudaGetErrorString(err));
     *flops = 2.0 * kProbeIters * kProbeChains * double(block) * double(grid);
     *milliseconds = ms;
+    return CBX_OK;
+}
+
+extern "C" int cbx_claim_order(const double* work, const double* scale, double exponent, long long n, long long* order,
+                               void* scratch, size_t scratch_bytes, void* stream) {
+    if (n < 0 || n > 4294967295LL) return fail(CBX_ERR_ARGUMENT, "cbx_claim_order takes 0 to 2^32 - 1 runs, got %lld", n);
+    if (n == 0) return CBX_OK;
+    if (!work || !order) return fail(CBX_ERR_ARGUMENT, "work and order are required");
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    const float e = (float)exponent;
+    if (n <= kOrderOneBlock) {
+        order_one_block_kernel<<<1, kOrderThreads, 0, st>>>(work, scale, e, (int)n, order);
+    } else {
+        if (!scratch || scratch_bytes < CBX_CLAIM_ORDER_SCRATCH_BYTES)
+            return fail(CBX_ERR_ARGUMENT, "cbx_claim_order needs %d bytes of scratch for %lld runs",
+                        CBX_CLAIM_ORDER_SCRATCH_BYTES, n);
+        static_assert(CBX_CLAIM_ORDER_SCRATCH_BYTES == 2 * kOrderBins * sizeof(unsigned), "scratch size");
+        unsigned* counts = static_cast<unsigned*>(scratch);
+        cudaError_t e0 = cudaMemsetAsync(scratch, 0, CBX_CLAIM_ORDER_SCRATCH_BYTES, st);
+        if (e0 != cudaSuccess) return fail(CBX_ERR_RUNTIME, "clearing the claim-order scratch: %s", cudaGetErrorString(e0));
+        const unsigned grid = (unsigned)((n + kOrderTile - 1) / kOrderTile);
+        order_count_kernel<<<grid, kOrderThreads, 0, st>>>(work, scale, e, n, counts);
+        order_scatter_kernel<<<grid, kOrderThreads, 0, st>>>(work, scale, e, n, counts, counts + kOrderBins, order);
+    }
+    cudaError_t err = cudaGetLastError();
+    if (err != cudaSuccess) return fail(CBX_ERR_RUNTIME, "claim-order launch: %s", cudaGetErrorString(err));
     return CBX_OK;
 }
 

@@ -733,13 +733,27 @@ class Solver:
         (an error-controlled step shrinks as the (q+1)-th root of the
         tolerance), so a long, tight run is not claimed after shorter,
         cheaper ones and left running alone at the end of the launch.
+        On the device, runs within a few percent of each other come in any
+        order (``cbx_claim_order``).
         Each run's result does not depend on the order."""
         if dur_t is None or self.schedule == "index" or self.launch_kind == 0:
             return None
         torch = _torch()
+        scaled = tol_t is not None and self.controller != "fixed"
+        q = max(int(getattr(self.tableau, "order", 1) or 1), 1)
+        n = int(dur_t.numel())
+        if dur_t.is_cuda and dur_t.dtype == torch.float64 and dur_t.dim() == 1 and dur_t.is_contiguous() \
+                and 0 < n < 2 ** 32:
+            order = torch.empty((n,), device=dur_t.device, dtype=torch.int64)
+            scratch = torch.empty((_native.CLAIM_ORDER_SCRATCH_BYTES // 4,), device=dur_t.device, dtype=torch.int32)
+            scale = tol_t.to(torch.float64).reshape(-1).contiguous() if scaled else None
+            with torch.cuda.device(dur_t.device):
+                _native.claim_order(dur_t.data_ptr(), None if scale is None else scale.data_ptr(), -1.0 / (q + 1), n,
+                                    order.data_ptr(), scratch.data_ptr(),
+                                    torch.cuda.current_stream(dur_t.device).cuda_stream)
+            return order
         cost = dur_t
-        if tol_t is not None and self.controller != "fixed":
-            q = max(int(getattr(self.tableau, "order", 1) or 1), 1)
+        if scaled:
             cost = dur_t * torch.clamp(tol_t, min=1e-300) ** (-1.0 / (q + 1))
         return torch.argsort(cost, descending=True).to(torch.int64).contiguous()
 

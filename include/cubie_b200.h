@@ -106,6 +106,16 @@ int cbx_fp32_peak_probe(int device, double* flops, float* milliseconds);
  * flush between timed launches). */
 int cbx_flush_l2(void* buffer, size_t bytes, void* stream);
 
+/* Claim order for a persistent launch (args->run_order): a permutation of
+ * [0, n) in ``order`` by decreasing work[i] * scale[i]^exponent (scale may be
+ * NULL), runs within about 4 % of each other in no particular order.  Device
+ * pointers; ``scratch`` of CBX_CLAIM_ORDER_SCRATCH_BYTES (contents
+ * arbitrary) may be NULL up to 4,096 runs.  Asynchronous on ``stream``,
+ * whose device must be current. */
+#define CBX_CLAIM_ORDER_SCRATCH_BYTES 16384
+int cbx_claim_order(const double* work, const double* scale, double exponent, long long n, long long* order,
+                    void* scratch, size_t scratch_bytes, void* stream);
+
 /* Discrete adjoint (no counterpart in the reference, which cannot
  * differentiate its integrations).  For a module generated with the
  * adjoint kernels (explicit Runge-Kutta and Rosenbrock tableaus):
