@@ -3,8 +3,8 @@
 // local memory).
 //
 // Layout: lane l of the warp holds components l, l + 32, l + 64, ... of
-// every state-sized vector (L = ceil(N / 32) values per lane, padded with
-// zeros).  The right-hand side and the Jacobian-vector product are
+// every state-sized vector, or the components the generated layout gives it
+// (L values per lane, padded with zeros).  The right-hand side and the Jacobian-vector product are
 // evaluated by the whole warp through generated functions
 // (cubie_b200/warpgen.py): per-lane code over registers and shuffles where
 // the system's couplings lie at constant offsets (``RegisterForm`` below),
@@ -46,16 +46,18 @@ __device__ __forceinline__ T warp_sum(T v) {
 // What bounds the kernel is the latency of those exchanges and the issue
 // slots of their loads and stores, not arithmetic or bandwidth.  Shared
 // against register form, Hodgkin-Huxley cables, l_stable_dirk_3 + BiCGSTAB,
-// 80 steps on one B200: 76 states x 5,003 runs 7.35 -> 3.33 ms, 256 x 1,536
-// 4.03 -> 1.44, 384 x 1,000 4.43 -> 1.56, 512 x 800 5.61 -> 2.27; FP64 256 x
+// 80 steps on one B200: 76 states x 5,003 runs 7.35 -> 2.60 ms, 256 x 1,536
+// 4.03 -> 1.33, 384 x 1,000 4.43 -> 1.37, 512 x 800 5.61 -> 2.03; FP64 256 x
 // 1,536 11.4 -> 8.6.  512 FP32 and 256 FP64 states (832 bytes a lane by the
 // count below) spill part of their vectors to local memory and still gain;
 // nothing larger was measured, so the rule ends there.
 template <class Cfg>
 struct RegisterForm {
-    static constexpr int L = (Cfg::N + 31) / 32;
-    static constexpr int BYTES = int(sizeof(typename Cfg::R)) * (10 * L + Cfg::WSys::NC);
+    static constexpr int BYTES = int(sizeof(typename Cfg::R)) * (10 * Cfg::WSys::SLOTS + Cfg::WSys::NC);
     static constexpr bool VALUE = Cfg::WSys::NC > 0 && BYTES <= 832;
+    // vector components per lane: the generated layout's slots (LaneMap), or
+    // the components in a row
+    static constexpr int L = VALUE ? Cfg::WSys::SLOTS : (Cfg::N + 31) / 32;
 };
 
 // Per-warp shared memory.  With a cached Jacobian (WSys::NNZ > 0) the
@@ -80,8 +82,8 @@ struct WarpMem {
     R ylin[CACHED ? 1 : N];               // linearisation point (matrix-free J v)
     R sbase[SH];                          // stage base state (shared placement)
     R sstart[SH];                         // step start state (shared placement)
-    R r0[Cfg::SHARED_SCRATCH ? 32 * ((N + 31) / 32) : 1];  // BiCGSTAB shadow residual (shared placement)
-    R sz[Cfg::SHARED_SCRATCH ? 32 * ((N + 31) / 32) : 1];  // stage increment in and out of the solve
+    R r0[Cfg::SHARED_SCRATCH ? 32 * RegisterForm<Cfg>::L : 1];  // BiCGSTAB shadow residual (shared placement)
+    R sz[Cfg::SHARED_SCRATCH ? 32 * RegisterForm<Cfg>::L : 1];  // stage increment in and out of the solve
     R p[Cfg::NP > 0 ? Cfg::NP : 1];
     R d[Cfg::ND > 0 ? Cfg::ND : 1];       // drivers of the evaluation
     R dlin[Cfg::ND > 0 ? Cfg::ND : 1];    // drivers at the linearisation point
@@ -91,7 +93,7 @@ template <class Cfg>
 struct WarpCtx {
     using R = typename Cfg::R;
     using C = typename Cfg::C;
-    static constexpr int N = Cfg::N, ND = Cfg::ND, L = (Cfg::N + 31) / 32;
+    static constexpr int N = Cfg::N, ND = Cfg::ND, L = RegisterForm<Cfg>::L;
     static constexpr bool CACHED = WarpMem<Cfg>::CACHED;
     static constexpr bool REG = WarpMem<Cfg>::REG;
     static constexpr int NC = REG ? Cfg::WSys::NC : 1;                     // register form: coefficients,
@@ -102,17 +104,24 @@ struct WarpCtx {
     C tol_scale;
     mutable R tlin;
 
-    // every slot is a component when N is a multiple of 32 (the check then
-    // folds away from every per-lane loop)
-    __device__ __forceinline__ bool valid(int k) const { return (N % 32 == 0) || lane + 32 * k < N; }
+    // whether slot k of the lane is a component (the check folds away from
+    // every per-lane loop where every lane holds one), and which
+    __device__ __forceinline__ bool valid(int k) const {
+        if constexpr (REG) return Cfg::WSys::slot_count(k) == 32 || lane < Cfg::WSys::slot_count(k);
+        else return (N % 32 == 0) || lane + 32 * k < N;
+    }
+    __device__ __forceinline__ int comp(int k) const {
+        if constexpr (REG) return Cfg::WSys::slot_base(k) + lane * Cfg::WSys::LANE_STRIDE;
+        else return lane + 32 * k;
+    }
     __device__ __forceinline__ void put(R* dst, const R* loc) const {
 #pragma unroll
         for (int k = 0; k < L; ++k)
-            if (valid(k)) dst[lane + 32 * k] = loc[k];
+            if (valid(k)) dst[comp(k)] = loc[k];
     }
     __device__ __forceinline__ void get(const R* src, R* loc) const {
 #pragma unroll
-        for (int k = 0; k < L; ++k) loc[k] = valid(k) ? src[lane + 32 * k] : R(0);
+        for (int k = 0; k < L; ++k) loc[k] = valid(k) ? src[comp(k)] : R(0);
     }
     __device__ __forceinline__ void put_drivers(R* dst, const R* drv) const {
 #pragma unroll
@@ -307,12 +316,12 @@ struct WarpDirkProblem {
     R J[WarpCtx<Cfg>::NC];                       // register form: coefficients at the last linearisation
     R kwr[WarpStageOp<Cfg>::KW];                 // and the stage solve's Krylov weights
     __device__ __forceinline__ R b(int k) const {
-        if constexpr (Cfg::SHARED_SCRATCH) return w.valid(k) ? w.m->sbase[w.lane + 32 * k] : R(0);
+        if constexpr (Cfg::SHARED_SCRATCH) return w.valid(k) ? w.m->sbase[w.comp(k)] : R(0);
         else if constexpr (Cfg::REG_SCRATCH) return base_v[k];
         else return base_p[k];
     }
     __device__ __forceinline__ R y0(int k) const {
-        if constexpr (Cfg::SHARED_SCRATCH) return w.valid(k) ? w.m->sstart[w.lane + 32 * k] : R(0);
+        if constexpr (Cfg::SHARED_SCRATCH) return w.valid(k) ? w.m->sstart[w.comp(k)] : R(0);
         else if constexpr (Cfg::REG_SCRATCH) return start_v[k];
         else return start_p[k];
     }
@@ -357,7 +366,7 @@ struct WarpDirkProblem {
         for (int k = 0; k < K; ++k) {
             if constexpr (WarpCtx<Cfg>::REG) kwr[k] = R(0);
             if (!w.valid(k)) continue;
-            const int c = w.lane + 32 * k;
+            const int c = w.comp(k);
             R v;
             if constexpr (Cfg::MIXED)
                 v = R(1) / max_nan(R(Cfg::katol(c)) + R(Cfg::krtol(c)) * R(w.tol_scale) * absv(b(k)), R(1e-16));
@@ -373,7 +382,7 @@ struct WarpDirkProblem {
 #pragma unroll
         for (int k = 0; k < K; ++k) {
             if (!w.valid(k)) continue;
-            const int c = w.lane + 32 * k;
+            const int c = w.comp(k);
             const R sv = b(k) + a * z[k];
             const R ref = max_nan(absv(sv), absv(y0(k)));
             const C ratio = tol_ratio<Cfg>(delta[k], ref, Cfg::natol(c), Cfg::nrtol(c), w.tol_scale);
@@ -488,9 +497,11 @@ struct WarpDirkStep {
             int2 it2;
             if constexpr (Cfg::SHARED_SCRATCH) {
                 w.put(w.m->sbase, base);
-                w.put(w.m->sz, ps.z);
+#pragma unroll
+                for (int k = 0; k < L; ++k) w.m->sz[w.lane + 32 * k] = ps.z[k];
                 st = stage_solve(w, nullptr, nullptr, drv_stage, stage_time, dt, a, nullptr, ps.theta, it2);
-                w.get(w.m->sz, ps.z);
+#pragma unroll
+                for (int k = 0; k < L; ++k) ps.z[k] = w.m->sz[w.lane + 32 * k];
             } else {
                 st = stage_solve(w, base, y, drv_stage, stage_time, dt, a, ps.z, ps.theta, it2);
             }
@@ -736,8 +747,7 @@ __device__ __forceinline__ void warp_begin(WarpLane<Cfg>& L, WarpCtx<Cfg>& w, co
     const R* params = static_cast<const R*>(a.params);
 #pragma unroll
     for (int k = 0; k < NL; ++k) {
-        const int c = w.lane + 32 * k;
-        L.y[k] = c < Cfg::N ? inits[c * a.run_stride + run] : R(0);
+        L.y[k] = w.valid(k) ? inits[w.comp(k) * a.run_stride + run] : R(0);
         L.comp[k] = R(0);
     }
 #pragma unroll
@@ -844,7 +854,7 @@ __device__ __forceinline__ bool warp_iterate(WarpLane<Cfg>& L, WarpCtx<Cfg>& w, 
 #pragma unroll
         for (int i = 0; i < NL; ++i) {
             if (!w.valid(i)) continue;
-            const int c = w.lane + 32 * i;
+            const int c = w.comp(i);
             const R e = step_failed ? R(1e16) : err[i];
             const C ratio = C(Ctl::error_ratio(e, ynew[i], L.y[i], G(Cfg::atol(c)), G(Cfg::rtol(c)), ts));
             nrm2 += ratio * ratio;
@@ -961,8 +971,14 @@ __device__ __forceinline__ void run_warp(const cbx_solve_args& a) {
 
 }  // namespace cbx
 
+// Launch bounds: the block size, plus a minimum of resident blocks where the
+// generator asks for one (kernelgen.warp_min_blocks).
+#ifndef CBX_WARP_BOUNDS
+#define CBX_WARP_BOUNDS(CFG) __launch_bounds__(CFG::BLOCK)
+#endif
+
 #define CBX_DEFINE_WARP_KERNEL(CFG)                                                                  \
     extern "C" __device__ char cbx_warp_smem_probe[sizeof(cbx::WarpMem<CFG>) * (CFG::BLOCK / 32)];      \
-    extern "C" __global__ void __launch_bounds__(CFG::BLOCK) cbx_integrate_warp(cbx_solve_args a) {    \
+    extern "C" __global__ void CBX_WARP_BOUNDS(CFG) cbx_integrate_warp(cbx_solve_args a) {    \
         cbx::run_warp<CFG>(a);                                                                         \
     }

@@ -418,6 +418,26 @@ def generate_hetero_kernel(families: Sequence[Tuple[SymbolicODE, KernelSpec, Gen
     return "\n".join(lines) + "\n"
 
 
+def warp_min_blocks(spec: KernelSpec, warp_code) -> int:
+    """Minimum of resident blocks per SM asked for the warp kernel's register
+    form (0: the compiler's own choice).
+
+    Left to itself the compiler gave the 256-state cable 168 or 212 registers
+    (12 or 8 resident warps; 1.33 or 1.79 ms) from one small change of the
+    source to the next.  Measured (cables, FP32 with FP64
+    control, 80 steps; its own choice / 12 warps / 16 warps): 160 states 2.55 /
+    2.52 / 2.63 ms, 176 2.31 / 2.31 / 1.83, 192 2.03 / 2.03 / 1.67, 224 1.46 /
+    1.48 / 1.90, 256 1.79 / 1.33 / 1.60, 288 2.56 / 2.14 / 2.77, 320 2.25 /
+    2.03 / 2.50, 384 1.37 / 1.96 / 2.60, 512 2.03 / 2.93 / 3.94: 16 warps
+    where the lane's vectors then just fit 128 registers, 12 where they fit
+    168, and no bound where it would spill them or is not needed."""
+    if not warp_code.register_slots or spec.max_registers:
+        return 0
+    nbytes = np.dtype(spec.precision).itemsize * (10 * warp_code.register_slots + warp_code.register_coefs)
+    warps = 16 if 300 < nbytes <= 360 else (12 if 360 < nbytes <= 540 else 0)
+    return warps * 32 // int(spec.block_size)
+
+
 def _generate_warp_kernel(system: SymbolicODE, spec: KernelSpec, gen: GeneratedSystem, warp_code=None):
     """Translation unit of the warp-per-system layout (``cbx_integrate_warp``)."""
     from .warpgen import generate_warp_system
@@ -434,6 +454,9 @@ def _generate_warp_kernel(system: SymbolicODE, spec: KernelSpec, gen: GeneratedS
     spec = replace(spec, dense_prediction=False)
     lines = ["// generated by cubie_b200.kernelgen (warp-per-system layout); do not edit",
              f"// register cap: {int(spec.max_registers)}"]
+    min_blocks = warp_min_blocks(spec, warp_code)
+    if min_blocks:
+        lines.append(f"#define CBX_WARP_BOUNDS(CFG) __launch_bounds__(CFG::BLOCK, {min_blocks})")
     lines += DEVICE_INCLUDES
     lines.append('#include "cbx_warp.cuh"')
     lines.append("namespace cbxsys {")

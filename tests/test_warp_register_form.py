@@ -20,6 +20,13 @@ def _ring(n):
     return eqs, states, {"k": 1.0}, []
 
 
+def _interleaved(n):
+    """The ring with its cells' variables side by side."""
+    eqs, states, params, drivers = _ring(n)
+    order = [f"{v}{i:03d}" for i in range(n) for v in "uw"]
+    return eqs, {k: states[k] for k in order}, params, drivers
+
+
 def _scattered(n):
     """No constant offsets: every component reads another, in no pattern."""
     rng = np.random.default_rng(5)
@@ -37,18 +44,20 @@ def _code(model):
     return sysm, generate_system(sysm), generate_warp_system(sysm)
 
 
-# one slot, a slot shared by several variables, an odd size, more than two
-# slots; a multiple of 32 and not; ends that wrap over the whole vector
-@pytest.mark.parametrize("model", [hh_cable(3), hh_cable(16), hh_cable(19), hh_cable(40), _ring(5), _ring(33)],
-                         ids=["cable3", "cable16", "cable19", "cable40", "ring5", "ring33"])
+# one slot, a slot shared by several variables, an odd size (a slot per
+# variable), more than two slots; a multiple of 32 and not; ends that wrap over
+# the whole vector; variables interleaved cell by cell
+@pytest.mark.parametrize("model", [hh_cable(3), hh_cable(16), hh_cable(19), hh_cable(40), _ring(5), _ring(33),
+                                   _interleaved(33), _interleaved(64)],
+                         ids=["cable3", "cable16", "cable19", "cable40", "ring5", "ring33", "interleaved33",
+                              "interleaved64"])
 def test_lanes_equal_straight_line_code(model, tmp_path):
     sysm, g, w = _code(model)
     assert "NC = 0" not in w.source
     n = sysm.num_states
-    slots = (n + 31) // 32
     src = ("#include <cmath>\n#define __device__\n#define __forceinline__ inline\n"
            "#define CBX_NOINLINE __attribute__((noinline))\nusing std::exp; using std::pow;\n"
-           + g.source + "\n" + w.source + f"\nconstexpr int L = {slots}, N = {n};\n" + r'''
+           + g.source + "\n" + w.source + f"\nconstexpr int L = WarpSystem::SLOTS;\n" + r'''
 using W = WarpSystem;
 static void gather(const double loc[32][L], double g[32][W::NG > 0 ? W::NG : 1]) {
     for (int lane = 0; lane < 32; ++lane)
@@ -61,7 +70,8 @@ static void gather(const double loc[32][L], double g[32][W::NG > 0 ? W::NG : 1])
 }
 static void spread(const double* a, double loc[32][L]) {
     for (int lane = 0; lane < 32; ++lane)
-        for (int k = 0; k < L; ++k) loc[lane][k] = lane + 32 * k < N ? a[lane + 32 * k] : 0.0;
+        for (int k = 0; k < L; ++k)
+            loc[lane][k] = lane < W::slot_count(k) ? a[W::slot_base(k) + lane * W::LANE_STRIDE] : 0.0;
 }
 extern "C" double eval(const double* y, const double* v, const double* p, const double* d, double* f1, double* j1,
                        double* f2, double* f3, double* j3) {
@@ -76,7 +86,8 @@ extern "C" double eval(const double* y, const double* v, const double* p, const 
         W::fj_reg<double>(yl[lane], gy[lane], p, d, 0.0, lane, fb, jc);
         W::jmv_reg<double>(vl[lane], gv[lane], jc, jv);
         for (int k = 0; k < L; ++k) {
-            if (lane + 32 * k < N) { f2[lane + 32 * k] = fa[k]; f3[lane + 32 * k] = fb[k]; j3[lane + 32 * k] = jv[k]; }
+            const int c = W::slot_base(k) + lane * W::LANE_STRIDE;
+            if (lane < W::slot_count(k)) { f2[c] = fa[k]; f3[c] = fb[k]; j3[c] = jv[k]; }
             else padding += std::fabs(fa[k]) + std::fabs(fb[k]) + std::fabs(jv[k]);
         }
     }
@@ -97,7 +108,7 @@ extern "C" double eval(const double* y, const double* v, const double* p, const 
     v = rng.normal(size=n)
     p = np.array([120.0, 36.0, 0.5])
     d = np.array([3.0])
-    f1, j1, f2, f3, j3 = (np.zeros(n) for _ in range(5))
+    f1, j1, f2, f3, j3 = (np.full(n, np.nan) for _ in range(5))   # every component is written
     padding = lib.eval(*[a.ctypes.data for a in (y, v, p, d, f1, j1, f2, f3, j3)])
     # the same expressions in another order of sums: a few roundings
     np.testing.assert_allclose(f2, f1, rtol=1e-13, atol=1e-12)
