@@ -97,7 +97,7 @@ EXPORTED = (
     "cbx_module_load", "cbx_module_create", "cbx_module_destroy", "cbx_kernel_info",
     "cbx_occupancy", "cbx_solve", "cbx_device_info", "cbx_fp32_peak_probe", "cbx_flush_l2",
     "cbx_solve_noalloc", "cbx_adjoint_info", "cbx_adjoint_tape_bytes", "cbx_adjoint_launch", "cbx_solve_hetero",
-    "cbx_claim_order",
+    "cbx_claim_order", "cbx_adjoint_launch_records",
 )
 
 _lib = None
@@ -161,6 +161,7 @@ def lib():
         L.cbx_adjoint_tape_bytes.argtypes = [ctypes.c_void_p, ctypes.POINTER(ctypes.c_longlong)]
         L.cbx_adjoint_launch.argtypes = [ctypes.c_void_p, ctypes.POINTER(SolveArgs), ctypes.POINTER(AdjointArgs),
                                          ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_void_p]
+        L.cbx_adjoint_launch_records.argtypes = L.cbx_adjoint_launch.argtypes
         _lib = L
         return L
 
@@ -274,9 +275,10 @@ class Module:
         return v.value
 
     def adjoint_launch(self, args: SolveArgs, adj: AdjointArgs, phase: int, block: int, grid: int = 0,
-                       stream: int = 0) -> None:
-        _check(lib().cbx_adjoint_launch(self._handle, ctypes.byref(args), ctypes.byref(adj), phase, block, grid,
-                                        ctypes.c_void_p(stream)), "cbx_adjoint_launch")
+                       stream: int = 0, records: bool = False) -> None:
+        name = "cbx_adjoint_launch_records" if records else "cbx_adjoint_launch"
+        _check(getattr(lib(), name)(self._handle, ctypes.byref(args), ctypes.byref(adj), phase, block, grid,
+                                    ctypes.c_void_p(stream)), name)
 
     def __del__(self):
         try:

@@ -17,10 +17,14 @@ tableaus for autonomous systems without drivers) gets two extra kernels (``csrc/
 :class:`AdjointIntegrator` drives the two launches;
 :func:`solve_ivp_adjoint` wraps them in a ``torch.autograd.Function`` so a
 torch loss on the returned state tensor back-propagates into the initial
-values and parameters.  Memory: ``n_runs * max_ckpts`` checkpoint images,
-one replay segment of ``ckpt_every`` records per run and, for explicit
-tableaus, ``n_runs * max_ckpts * ckpt_every`` tape entries
-(:meth:`AdjointIntegrator.sizes` gives the three sizes in bytes).  A run that
+values and parameters.  While every run has a lane of its own and a
+record (start state and size) of every accepted step of every run fits
+``record_share`` of the device's memory, the forward launch stores those instead of checkpoints and the backward
+launch reads them without replaying anything.  Memory:
+``n_runs * max_ckpts * ckpt_every`` records, or ``n_runs * max_ckpts``
+checkpoint images, one replay segment of ``ckpt_every`` records per run and,
+for explicit tableaus, ``n_runs * max_ckpts * ckpt_every`` tape entries
+(:meth:`AdjointIntegrator.sizes` gives the sizes in bytes).  A run that
 needs more than ``max_ckpts * ckpt_every`` accepted steps stops with
 status 32 (step budget), like ``max_steps``.
 """
@@ -38,7 +42,7 @@ from .solver import Solver, _torch
 class AdjointIntegrator:
     """Forward-with-checkpoints and reverse sweeps for one solver."""
 
-    def __init__(self, solver: Solver, ckpt_every: int = 64, max_ckpts: int = 64):
+    def __init__(self, solver: Solver, ckpt_every: int = 64, max_ckpts: int = 64, record_share: float = 0.125):
         if not solver.adjoint:
             raise ValueError("build the Solver with adjoint=True")
         if not solver.output_types or "state" not in solver.output_types:
@@ -48,6 +52,25 @@ class AdjointIntegrator:
         self.solver = solver
         self.ckpt_every = int(ckpt_every)
         self.max_ckpts = int(max_ckpts)
+        self.record_share = float(record_share)
+
+    def _records(self, n_runs: int, record: int, dev):
+        """Buffer for a record of every step (``max_ckpts * ckpt_every`` per
+        run), or None where checkpoints and replay are used instead: more
+        runs than the device has lanes for at once (1,024 an SM at these
+        kernels' registers; cbx_adjoint.cuh has the times), or records above
+        ``record_share`` of the device's memory or of what is free."""
+        torch = _torch()
+        device = torch.cuda.get_device_properties(dev)
+        cap = self.max_ckpts * self.ckpt_every
+        nbytes = n_runs * cap * record
+        if (n_runs > 1024 * device.multi_processor_count or cap >= 2 ** 31
+                or nbytes > self.record_share * device.total_memory):
+            return None
+        try:
+            return torch.empty((max(nbytes, 16) // 4,), device=dev, dtype=torch.int32)
+        except torch.cuda.OutOfMemoryError:
+            return None
 
     def sizes(self, prep) -> tuple:
         """(bytes of one checkpoint image, bytes of one replay record, bytes
@@ -73,6 +96,11 @@ class AdjointIntegrator:
             adj.tape = adj.tape_flags = adj.step_count = None
         else:
             adj.tape, adj.tape_flags, adj.step_count = (t.data_ptr() for t in tape)
+
+    @staticmethod
+    def _set_records(adj, records, steps, n_runs: int) -> None:
+        if records is not None:
+            adj.seg, adj.step_count, adj.lane_words = records.data_ptr(), steps.data_ptr(), n_runs
 
     def forward(self, inits_t, params_t, duration: float, settling_time: float = 0.0, t0: float = 0.0,
                 stream=None, tol_scale=None):
@@ -101,20 +129,26 @@ class AdjointIntegrator:
         lane, record, tape_entry = self.sizes(prep)
         words = lane // 4
         with torch.cuda.stream(st):
-            ckpt = torch.empty((n_runs * self.max_ckpts * words,), device=dev, dtype=torch.int32)
+            records = self._records(n_runs, record, dev)
             count = torch.zeros((n_runs,), device=dev, dtype=torch.int32)
-            tape = self._tape_buffers(n_runs, tape_entry, dev) if tape_entry > 0 else None
+            ckpt = tape = steps = None
+            if records is not None:
+                steps = torch.empty((n_runs,), device=dev, dtype=torch.int32)
+            else:
+                ckpt = torch.empty((n_runs * self.max_ckpts * words,), device=dev, dtype=torch.int32)
+                tape = self._tape_buffers(n_runs, tape_entry, dev) if tape_entry > 0 else None
         adj = _native.AdjointArgs()
-        adj.ckpt = ckpt.data_ptr()
+        adj.ckpt = None if ckpt is None else ckpt.data_ptr()
         adj.ckpt_count = count.data_ptr()
         adj.lane_words = words
         adj.ckpt_every = self.ckpt_every
         adj.max_ckpts = self.max_ckpts
         self._set_tape(adj, tape)
-        prep["module"].adjoint_launch(args, adj, 0, s.block_size, 0, st.cuda_stream)
+        self._set_records(adj, records, steps, n_runs)
+        prep["module"].adjoint_launch(args, adj, 0, s.block_size, 0, st.cuda_stream, records is not None)
         saved = dict(prep=prep, bufs=bufs, inits=inits_t, params=params_t, tol=tol_t, ckpt=ckpt, count=count,
                      words=words,
-                     record=record, tape=tape,
+                     record=record, tape=tape, records=records, steps=steps,
                      n_runs=n_runs, duration=duration, settling_time=settling_time, t0=t0, dev=dev, tdtype=tdtype)
         return bufs["state"], bufs["status"], saved
 
@@ -135,15 +169,17 @@ class AdjointIntegrator:
         st = stream if stream is not None else torch.cuda.current_stream(dev)
         st.wait_stream(torch.cuda.current_stream(dev))
         with torch.cuda.stream(st):
-            seg = torch.empty((self.ckpt_every * n_runs * saved["record"] // 4,), device=dev, dtype=torch.int32)
+            seg = None
+            if saved["records"] is None:
+                seg = torch.empty((self.ckpt_every * n_runs * saved["record"] // 4,), device=dev, dtype=torch.int32)
             gi = torch.empty((n, n_runs), device=dev, dtype=tdtype)
             gp = torch.empty((max(npar, 1), n_runs), device=dev, dtype=tdtype)
             args = s.make_args(prep, bufs, saved["inits"], saved["params"], None, n_runs, saved["duration"],
                                saved["settling_time"], saved["t0"], None, saved["tol"])  # zeroes the work counter
         adj = _native.AdjointArgs()
-        adj.ckpt = saved["ckpt"].data_ptr()
+        adj.ckpt = None if saved["ckpt"] is None else saved["ckpt"].data_ptr()
         adj.ckpt_count = saved["count"].data_ptr()
-        adj.seg = seg.data_ptr()
+        adj.seg = None if seg is None else seg.data_ptr()
         adj.grad_state = grad_state.data_ptr()
         adj.grad_inits = gi.data_ptr()
         adj.grad_params = gp.data_ptr() if npar > 0 else None
@@ -151,7 +187,8 @@ class AdjointIntegrator:
         adj.ckpt_every = self.ckpt_every
         adj.max_ckpts = self.max_ckpts
         self._set_tape(adj, saved["tape"])
-        prep["module"].adjoint_launch(args, adj, 1, s.block_size, 0, st.cuda_stream)
+        self._set_records(adj, saved["records"], saved["steps"], n_runs)
+        prep["module"].adjoint_launch(args, adj, 1, s.block_size, 0, st.cuda_stream, saved["records"] is not None)
         return gi, (gp if npar > 0 else gp[:0])
 
 
@@ -165,7 +202,10 @@ def _function():
         def forward(ctx, inits, params, integ, duration, settling_time, t0):
             state, status, saved = integ.forward(inits, params, duration, settling_time, t0)
             ctx.integ = integ
-            ctx.saved = saved
+            # the output carries this node: kept by an alias here, or output and
+            # node would hold each other (and the records) until the cycle
+            # collector runs
+            ctx.saved = dict(saved, bufs=dict(saved["bufs"], state=state.detach()))
             ctx.in_dtypes = (inits.dtype, params.dtype)
             ctx.mark_non_differentiable(status)
             return state, status

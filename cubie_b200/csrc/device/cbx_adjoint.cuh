@@ -778,6 +778,169 @@ __device__ __forceinline__ void run_adjoint_backward(const cbx_solve_args a, con
     }
 }
 
+// The record form: where memory allows a record of every accepted step of
+// every run (16 bytes for up to three FP32 states), the forward launch writes
+// them as it goes and the reverse sweep reads them back, so nothing is
+// replayed and no checkpoint or tape exists.  The records are those the
+// replay would produce (the forward's own step starts and sizes).
+//
+// The host uses it while every run has a lane of its own.  The lanes of a
+// warp then walk their steps side by side, and with the runs of one step
+// together ([step][run]) a warp's records are whole lines.  (A run's records
+// together cost a sector per lane and store, 84 us more on the forward
+// below.)  With more runs than lanes the lanes are at different steps, every
+// layout scatters, and the forward's stores cost more than the replay.
+// Checkpoints against records, forward + backward: FitzHugh-Nagumo, 131,072
+// runs x 130 steps, 1.29 -> 0.98 ms (5,000 runs 0.56 -> 0.48); Van der Pol
+// under ROS3P, 8,191 runs, 1.09 -> 0.89; 300,001 FitzHugh-Nagumo runs 2.35
+// against 2.57, 200,000 Van der Pol runs 3.95 against 4.25 (checkpoints kept).
+template <class Cfg>
+struct RecordWriter {
+    using R = typename Cfg::R;
+    using C = typename Cfg::C;
+    using Rec = SegRecord<Cfg>;
+    static constexpr bool ACTIVE = true;
+    R* next;
+    long long step_step;
+    int count;
+    __device__ __forceinline__ void accepted(const Lane<Cfg>& L, C dt_eff, int row) {
+        R rec[Rec::F];
+#pragma unroll
+        for (int k = 0; k < Cfg::N; ++k) rec[k] = L.y[k];
+        if constexpr (Rec::TIMED) rec[Rec::T_AT] = R(L.tp);
+        const R h = R(dt_eff);
+        rec[Rec::H_AT] = row >= 0 ? -h : h;
+#pragma unroll
+        for (int k = Rec::H_AT + 1; k < Rec::F; ++k) rec[k] = R(0);
+        Rec::store(next, rec);
+        next += step_step;
+        ++count;
+    }
+};
+
+template <class Cfg>
+__device__ __forceinline__ void run_adjoint_forward_records(const cbx_solve_args a, const cbx_adjoint_args g) {
+    using R = typename Cfg::R;
+    __shared__ BlockTotals bt;
+    totals_begin(&bt);
+    Lane<Cfg> L;
+    bool active = false, exhausted = false;
+    const int cap = g.max_ckpts * g.ckpt_every;
+    const long long step_step = g.lane_words * SegRecord<Cfg>::F;   // values from a run's record to its next
+    RecordWriter<Cfg> rec{nullptr, step_step, 0};
+    while (true) {
+        if (!active && !exhausted) {
+            const long long run = claim_run(a.work_counter);
+            if (run < a.n_runs) {
+                lane_begin<Cfg>(L, a, run);
+                active = true;
+                rec.next = static_cast<R*>(g.seg) + run * SegRecord<Cfg>::F;
+                rec.count = 0;
+            } else {
+                exhausted = true;
+            }
+        }
+        if (!__any_sync(0xffffffffu, active)) break;
+        if (active) {
+            bool done = false;
+            if (rec.count == cap) {
+                L.status |= MAX_LOOP_ITERS_EXCEEDED;
+                done = true;
+            } else {
+                done = lane_iterate<Cfg, RecordWriter<Cfg>>(L, a, &rec);
+            }
+            if (done) {
+                g.step_count[L.run] = rec.count;
+                g.ckpt_count[L.run] = L.save_idx;
+                lane_end<Cfg>(L, a, &bt);
+                active = false;
+            }
+        }
+    }
+    totals_flush(&bt, a);
+}
+
+// Reverse sweep over the records: every lane walks its own run backwards, the
+// next (earlier) record and the next saved row's loss gradient in flight.
+template <class Cfg>
+__device__ __forceinline__ void run_adjoint_backward_records(const cbx_solve_args a, const cbx_adjoint_args g) {
+    using R = typename Cfg::R;
+    using C = typename Cfg::C;
+    using Adj = StepAdjoint<Cfg, Cfg::ALGO>;
+    using Rec = SegRecord<Cfg>;
+    constexpr int N = Cfg::N, NP = Cfg::NP, F = Rec::F, NPP = NP > 0 ? NP : 1;
+    const long long s = a.run_stride;
+    const long long step_step = g.lane_words * F;
+    const R* params = static_cast<const R*>(a.params);
+    R lam[N], p[NPP], nxt[F];
+    C pbar[NPP];
+    C tol_scale = C(1);
+    RowGrad<Cfg> row_next;
+    long long run = -1;
+    const R* rec_at = nullptr;   // the record in ``nxt``
+    int j = -1, rows_end = 0;
+    bool active = false, exhausted = false;
+    while (true) {
+        if (!active && !exhausted) {
+            run = claim_run(a.work_counter);
+            if (run < a.n_runs) {
+                active = true;
+#pragma unroll
+                for (int q = 0; q < N; ++q) lam[q] = R(0);
+#pragma unroll
+                for (int q = 0; q < NPP; ++q) {
+                    pbar[q] = C(0);
+                    p[q] = NP > 0 ? params[q * s + run] : R(0);
+                }
+                tol_scale = a.tol_scale ? C(a.tol_scale[run]) : C(1);
+                j = g.step_count[run] - 1;
+                rows_end = g.ckpt_count[run];
+                if (j >= 0) {
+                    rec_at = static_cast<const R*>(g.seg) + run * F + j * step_step;
+                    Rec::load(rec_at, nxt);
+                    row_next.load(a, g, rows_end - 1, run);
+                }
+            } else {
+                exhausted = true;
+            }
+        }
+        if (!__any_sync(0xffffffffu, active)) break;
+        if (active && j >= 0) {
+            R rec_j[F];
+#pragma unroll
+            for (int k = 0; k < F; ++k) rec_j[k] = nxt[k];
+            if (j > 0) {
+                rec_at -= step_step;
+                Rec::load(rec_at, nxt);
+            }
+            const R hs = rec_j[Rec::H_AT];
+            if (hs < R(0)) {
+                row_next.add_to(lam);
+                --rows_end;
+                if (j > 0) row_next.load(a, g, rows_end - 1, run);
+            }
+            const R t = Rec::TIMED ? rec_j[Rec::T_AT] : R(0);
+            StepCtx<Cfg> ctx{p, static_cast<const R*>(a.driver_coeffs), tol_scale};
+            Adj::reverse(ctx, rec_j, t, fabs(hs), lam, pbar);
+            --j;
+        }
+        if (active && j < 0) {
+            if (a.warmup == 0.0) add_row_grad<Cfg>(lam, a, g, 0, run);
+            R* gi = static_cast<R*>(g.grad_inits);
+#pragma unroll
+            for (int q = 0; q < N; ++q) gi[q * s + run] = lam[q];
+            if constexpr (NP > 0) {
+                R* gp = static_cast<R*>(g.grad_params);
+                if (gp) {
+#pragma unroll
+                    for (int q = 0; q < NP; ++q) gp[q * s + run] = R(pbar[q]);
+                }
+            }
+            active = false;
+        }
+    }
+}
+
 }  // namespace cbx
 
 #define CBX_DEFINE_ADJOINT_KERNELS(CFG)                                                              \
@@ -791,4 +954,12 @@ __device__ __forceinline__ void run_adjoint_backward(const cbx_solve_args a, con
     extern "C" __global__ void CBX_LAUNCH_BOUNDS(CFG) cbx_adjoint_backward(cbx_solve_args a,          \
                                                                           cbx_adjoint_args g) {      \
         cbx::run_adjoint_backward<CFG>(a, g);                                                         \
+    }                                                                                                 \
+    extern "C" __global__ void CBX_LAUNCH_BOUNDS(CFG) cbx_adjoint_forward_records(cbx_solve_args a,    \
+                                                                                 cbx_adjoint_args g) { \
+        cbx::run_adjoint_forward_records<CFG>(a, g);                                                  \
+    }                                                                                                 \
+    extern "C" __global__ void CBX_LAUNCH_BOUNDS(CFG) cbx_adjoint_backward_records(cbx_solve_args a,   \
+                                                                                  cbx_adjoint_args g) { \
+        cbx::run_adjoint_backward_records<CFG>(a, g);                                                 \
     }

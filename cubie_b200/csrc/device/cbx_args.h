@@ -73,6 +73,12 @@ typedef struct cbx_solve_args {
  *               row), tape_flags [run][ceil(cap / 32)] 32-bit words (bit set:
  *               the attempt before that step was rejected), step_count [run]
  *               int32 (accepted steps).
+ *
+ * The record form (cbx_adjoint_launch_records) uses seg, step_count,
+ * ckpt_count and the gradient pointers only: the forward launch stores one
+ * record per accepted step, seg [cap][lane_words][record_bytes] with
+ * lane_words >= n_runs, and in ckpt_count the rows each run saved; the
+ * reverse sweep reads them and replays nothing.
  */
 typedef struct cbx_adjoint_args {
     void* ckpt;

@@ -29,7 +29,7 @@ struct cbx_module {
     int sm_count;
     // discrete-adjoint kernels, resolved on first use (modules generated
     // without them have neither)
-    CUfunction adj[2];
+    CUfunction adj[4];  // forward, backward, and both again in the record form
     size_t lane_bytes;
     size_t record_bytes;
     size_t tape_bytes;
@@ -477,8 +477,9 @@ int resolve_adjoint(cbx_module* m) {
     size_t rbytes = 0;
     if (g_drv.cuModuleGetGlobal(&probe2, &rbytes, m->module, "cbx_seg_record_probe") != CUDA_SUCCESS)
         return fail(CBX_ERR_ARGUMENT, "module was generated without the adjoint kernels");
-    const char* names[2] = {"cbx_adjoint_forward", "cbx_adjoint_backward"};
-    for (int k = 0; k < 2; ++k) {
+    const char* names[4] = {"cbx_adjoint_forward", "cbx_adjoint_backward", "cbx_adjoint_forward_records",
+                            "cbx_adjoint_backward_records"};
+    for (int k = 0; k < 4; ++k) {
         int rc = check_cu(g_drv.cuModuleGetFunction(&m->adj[k], m->module, names[k]), names[k]);
         if (rc) return rc;
     }
@@ -513,8 +514,9 @@ extern "C" int cbx_adjoint_tape_bytes(cbx_module* module, long long* entry_bytes
     return CBX_OK;
 }
 
-extern "C" int cbx_adjoint_launch(cbx_module* module, const cbx_solve_args* args, const cbx_adjoint_args* adj,
-                                  int phase, int block, int grid, void* stream) {
+namespace {
+int adjoint_launch(cbx_module* module, const cbx_solve_args* args, const cbx_adjoint_args* adj, bool records,
+                   int phase, int block, int grid, void* stream) {
     if (!module || !args || !adj) return fail(CBX_ERR_ARGUMENT, "null module, args or adjoint args");
     if (phase != 0 && phase != 1) return fail(CBX_ERR_ARGUMENT, "phase must be 0 (forward) or 1 (backward)");
     if (block <= 0 || block > 1024 || (block % 32) != 0)
@@ -523,11 +525,18 @@ extern "C" int cbx_adjoint_launch(cbx_module* module, const cbx_solve_args* args
         return fail(CBX_ERR_ARGUMENT, "run_stride (%lld) must be >= n_runs (%lld)", args->run_stride, args->n_runs);
     if (!args->inits || !args->work_counter)
         return fail(CBX_ERR_ARGUMENT, "inits and a zeroed work_counter are required");
-    if (!adj->ckpt || !adj->ckpt_count || adj->ckpt_every < 1 || adj->max_ckpts < 1)
+    if ((!adj->ckpt && !records) || !adj->ckpt_count || adj->ckpt_every < 1 || adj->max_ckpts < 1)
         return fail(CBX_ERR_ARGUMENT, "checkpoint buffers, ckpt_every >= 1 and max_ckpts >= 1 are required");
     if (phase == 0 && !args->status_out) return fail(CBX_ERR_ARGUMENT, "status_out is required");
     if (phase == 1 && (!adj->seg || !adj->grad_inits))
         return fail(CBX_ERR_ARGUMENT, "seg and grad_inits are required for the backward sweep");
+    if (records && (!adj->step_count || !adj->seg || (reinterpret_cast<size_t>(adj->seg) & 15) ||
+                    (long long)adj->ckpt_every * adj->max_ckpts > 2147483647LL))
+        return fail(CBX_ERR_ARGUMENT, "the record form needs 16-byte aligned records in seg, step_count, and at most "
+                    "2^31 - 1 records per run");
+    if (records && adj->lane_words < args->n_runs)
+        return fail(CBX_ERR_ARGUMENT, "the record form needs lane_words (%lld, runs per step) >= n_runs (%lld)",
+                    adj->lane_words, args->n_runs);
     if (!load_driver()) return fail(CBX_ERR_NO_DEVICE, "CUDA driver library is not available");
     CUcontext cur = nullptr;
     g_drv.cuCtxGetCurrent(&cur);
@@ -537,14 +546,14 @@ extern "C" int cbx_adjoint_launch(cbx_module* module, const cbx_solve_args* args
     }
     int rc = resolve_adjoint(module);
     if (rc) return rc;
-    if (module->tape_bytes > 0 && (!adj->tape || !adj->tape_flags || !adj->step_count))
+    if (!records && module->tape_bytes > 0 && (!adj->tape || !adj->tape_flags || !adj->step_count))
         return fail(CBX_ERR_ARGUMENT, "this module's adjoint needs a step-size tape, its flag words and step "
                     "counts (%zu bytes per entry)", module->tape_bytes);
-    if ((size_t)adj->lane_words * 4 < module->lane_bytes)
+    if (!records && (size_t)adj->lane_words * 4 < module->lane_bytes)
         return fail(CBX_ERR_ARGUMENT, "lane_words (%lld) is smaller than the module's lane image (%zu bytes)",
                     adj->lane_words, module->lane_bytes);
     if (args->n_runs == 0) return CBX_OK;
-    CUfunction f = module->adj[phase];
+    CUfunction f = module->adj[phase + (records ? 2 : 0)];
     long long g = grid;
     if (g <= 0) {
         int per_sm = 0;
@@ -561,6 +570,18 @@ extern "C" int cbx_adjoint_launch(cbx_module* module, const cbx_solve_args* args
     return check_cu(g_drv.cuLaunchKernel(f, (unsigned)g, 1, 1, (unsigned)block, 1, 1, 0,
                                          static_cast<CUstream>(stream), params, nullptr),
                     "cuLaunchKernel");
+}
+
+}  // namespace
+
+extern "C" int cbx_adjoint_launch(cbx_module* module, const cbx_solve_args* args, const cbx_adjoint_args* adj,
+                                  int phase, int block, int grid, void* stream) {
+    return adjoint_launch(module, args, adj, false, phase, block, grid, stream);
+}
+
+extern "C" int cbx_adjoint_launch_records(cbx_module* module, const cbx_solve_args* args,
+                                          const cbx_adjoint_args* adj, int phase, int block, int grid, void* stream) {
+    return adjoint_launch(module, args, adj, true, phase, block, grid, stream);
 }
 
 // ---------------------------------------------------------------------------

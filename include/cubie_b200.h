@@ -139,11 +139,18 @@ int cbx_claim_order(const double* work, const double* scale, double exponent, lo
  * dL/d(saved state) in adj->grad_state and args->work_counter zeroed
  * again, writes dL/d(initial state) and dL/d(parameters) for every run,
  * holding the accepted step sizes fixed.  Both are asynchronous on
- * ``stream``; grid = 0 picks a resident grid. */
+ * ``stream``; grid = 0 picks a resident grid.
+ *
+ * cbx_adjoint_launch_records does the same from a record of every accepted
+ * step (adj->seg, 16-byte aligned, max_ckpts * ckpt_every * lane_words *
+ * record_bytes with adj->lane_words >= n_runs): no checkpoints and no tape (those pointers are unused),
+ * the same step limit and the same gradients. */
 int cbx_adjoint_info(cbx_module* module, long long* lane_bytes, long long* record_bytes);
 int cbx_adjoint_tape_bytes(cbx_module* module, long long* entry_bytes);
 int cbx_adjoint_launch(cbx_module* module, const cbx_solve_args* args, const cbx_adjoint_args* adj,
                        int phase, int block, int grid, void* stream);
+int cbx_adjoint_launch_records(cbx_module* module, const cbx_solve_args* args, const cbx_adjoint_args* adj,
+                               int phase, int block, int grid, void* stream);
 
 /* Size of the device scratch array behind cbx_solve_noalloc.  Every device
  * that loads this library holds it until the process exits. */

@@ -1,0 +1,137 @@
+"""The adjoint's record form (a record of every accepted step, nothing
+replayed) against its checkpoint form: the records are the replay's own, so
+statuses and step limits are the same and the gradients agree to the
+roundings a separately compiled kernel may contract differently."""
+
+import ctypes
+import sys
+from pathlib import Path
+
+import numpy as np
+import pytest
+
+sys.path.insert(0, str(Path(__file__).resolve().parent / "host_emu"))
+
+FHN = ["dV = V - V**3 / 3 - w + I", "dw = (V + a - b * w) / tau"]
+VDP = ["dx = y", "dy = mu * (1 - x**2) * y - x"]
+DRIVER = r"""
+extern "C" void emu_records(cbx_solve_args* a, cbx_adjoint_args* g, int phase, int block) {
+    blockDim = {(unsigned)block, 1, 1};
+    gridDim = {1, 1, 1};
+    blockIdx = {0, 0, 0};
+    for (int t = 0; t < block; ++t) {
+        threadIdx = {(unsigned)t, 0, 0};
+        if (phase == 0) cbx_adjoint_forward_records(*a, *g);
+        else cbx_adjoint_backward_records(*a, *g);
+    }
+}
+"""
+
+
+def _solver(name, precision=np.float32, mixed=True):
+    from cubie_b200 import Solver, create_ODE_system
+    kw = dict(rtol=1e-5, atol=1e-5, output_types=["state"], save_every=1.0, adjoint=True, mixed_precision=mixed)
+    if name == "fhn":
+        sysm = create_ODE_system(FHN, states=["V", "w"], parameters=["a", "b", "tau", "I"], precision=precision)
+        return Solver(sysm, algorithm="dormand-prince-54", **kw)
+    sysm = create_ODE_system(VDP, states=["x", "y"], parameters=["mu"], precision=precision)
+    return Solver(sysm, algorithm="ros3p", linear_correction_type="direct", preconditioner_type=None, **kw)
+
+
+def _batch(name, n, seed=0):
+    rng = np.random.default_rng(seed)
+    if name == "fhn":
+        return (np.stack([rng.uniform(1, 2, n), rng.uniform(-0.5, 0.5, n)]),
+                np.stack([rng.uniform(0.6, 0.8, n), rng.uniform(0.7, 0.9, n), rng.uniform(8, 13, n),
+                          rng.uniform(0.5, 0.7, n)]))
+    return np.stack([rng.uniform(1, 2, n), rng.uniform(-1, 1, n)]), rng.uniform(0.5, 3.0, (1, n))
+
+
+@pytest.mark.parametrize("name", ["fhn", "vdp"])
+def test_emulated_records_equal_replay(name):
+    from emu import compile_emulated, run_emulated_adjoint
+    from cubie_b200 import _native
+    s = _solver(name)
+    x0, p = _batch(name, 5)
+    T, every, ckpts = 6.0, 4, 64
+    state, status, gi, gp = run_emulated_adjoint(s, x0, p, T, lambda y: 0.1 * y, every, ckpts)
+    prep = s.prepare(T, 0.0, 0.0, None, None, load=False)
+    lib = compile_emulated(prep["gen"].source + DRIVER)
+    n, cap = x0.shape[1], every * ckpts
+    x, q = np.ascontiguousarray(x0, np.float32), np.ascontiguousarray(p, np.float32)
+    out = dict(state=np.zeros_like(state), status=np.zeros_like(status), work=np.zeros(2, np.uint64),
+               seg=np.zeros(n * cap * int(lib.emu_record_bytes()) // 8 + 2), count=np.zeros(n, np.int32),
+               steps=np.zeros(n, np.int32), gi=np.zeros_like(gi), gp=np.zeros((p.shape[0], n), np.float32))
+    grad = np.ascontiguousarray(0.1 * state, np.float32)
+    a = _native.SolveArgs()
+    a.inits, a.params, a.state_out = x.ctypes.data, q.ctypes.data, out["state"].ctypes.data
+    a.status_out, a.work_counter = out["status"].ctypes.data, out["work"].ctypes.data
+    a.n_runs = a.run_stride = n
+    a.duration, a.save_stop, a.summary_stop = T, float(prep["save_stop"]), float(prep["summary_stop"])
+    a.n_save_rows = int(prep["n_save"])
+    g = _native.AdjointArgs()
+    g.seg, g.ckpt_count, g.step_count = (out[k].ctypes.data for k in ("seg", "count", "steps"))
+    g.ckpt_every, g.max_ckpts = every, ckpts
+    g.lane_words = n
+    g.grad_state, g.grad_inits, g.grad_params = grad.ctypes.data, out["gi"].ctypes.data, out["gp"].ctypes.data
+    lib.emu_records(ctypes.byref(a), ctypes.byref(g), 0, 32)
+    out["work"][:] = 0
+    lib.emu_records(ctypes.byref(a), ctypes.byref(g), 1, 32)
+    # one compiler, no contraction: the same bits
+    assert out["steps"].min() > 2 * every
+    np.testing.assert_array_equal(out["state"], state)
+    np.testing.assert_array_equal(out["status"], status)
+    np.testing.assert_array_equal(out["gi"], gi)
+    np.testing.assert_array_equal(out["gp"], gp)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name,precision,mixed,n", [("fhn", np.float32, True, 1001), ("fhn", np.float64, False, 33),
+                                                    ("vdp", np.float32, True, 1), ("vdp", np.float32, True, 777),
+                                                    ("fhn", np.float32, True, 151553)])   # more runs than lanes
+@pytest.mark.parametrize("every,ckpts", [(64, 64), (7, 90), (3, 4)])
+def test_records_equal_checkpoints(cuda_device, name, precision, mixed, n, every, ckpts):
+    import torch
+    from cubie_b200.adjoint import AdjointIntegrator
+    s = _solver(name, precision, mixed)
+    x0, p = (torch.tensor(v.astype(precision), device="cuda") for v in _batch(name, n, 3))
+    out = []
+    for share in (0.125, 0.0):
+        integ = AdjointIntegrator(s, ckpt_every=every, max_ckpts=ckpts, record_share=share)
+        state, status, saved = integ.forward(x0, p, 8.0)
+        assert (saved["records"] is not None) == (share > 0 and n < 151553)
+        out.append((state.clone(), status.clone(), *integ.backward(saved, 0.1 * state)))
+    (sa, ta, ga, pa), (sb, tb, gb, pb) = out
+    assert torch.equal(ta, tb)
+    if every * ckpts == 12:
+        assert bool((ta != 0).any())          # runs that reach the step limit stop alike
+    # the step is one function in both kernels; a contraction chosen
+    # differently is a rounding per operation, amplified over some hundred
+    # steps by the flow's own sensitivity (below 100 on these windows)
+    tol = 100 * 200 * (1.2e-7 if precision == np.float32 else 2.3e-16)
+    for u, v in ((sa, sb), (ga, gb), (pa, pb)):
+        assert float((u - v).norm()) <= tol * float(v.norm())
+
+
+@pytest.mark.gpu
+def test_autograd_passes_release_their_records(cuda_device):
+    import gc
+    import torch
+    from cubie_b200.adjoint import AdjointIntegrator, solve_ivp_adjoint
+    s = _solver("fhn")
+    x0, p = (torch.tensor(v.astype(np.float32), device="cuda") for v in _batch("fhn", 500, 3))
+    integ = AdjointIntegrator(s, 64, 64)
+    used = []
+    gc.collect()
+    gc.disable()
+    try:
+        for _ in range(3):
+            q = p.clone().requires_grad_(True)
+            state, status = solve_ivp_adjoint(s, x0.clone().requires_grad_(True), q, 8.0, integrator=integ)
+            (state ** 2).mean().backward()
+            assert bool(torch.isfinite(q.grad).all())
+            del state, status, q
+            used.append(torch.cuda.memory_allocated())
+    finally:
+        gc.enable()
+    assert used[1] == used[0] and used[2] == used[0]
