@@ -841,20 +841,22 @@ __device__ __forceinline__ void run_adjoint_forward_records(const cbx_solve_args
             }
         }
         if (!__any_sync(0xffffffffu, active)) break;
-        if (active) {
-            bool done = false;
-            if (rec.count == cap) {
-                L.status |= MAX_LOOP_ITERS_EXCEEDED;
-                done = true;
-            } else {
-                done = lane_iterate<Cfg, RecordWriter<Cfg>>(L, a, &rec);
+        bool done = false;
+        do {
+            if (active) {
+                if (rec.count == cap) {
+                    L.status |= MAX_LOOP_ITERS_EXCEEDED;
+                    done = true;
+                } else {
+                    done = lane_iterate<Cfg, RecordWriter<Cfg>>(L, a, &rec);
+                }
             }
-            if (done) {
-                g.step_count[L.run] = rec.count;
-                g.ckpt_count[L.run] = L.save_idx;
-                lane_end<Cfg>(L, a, &bt);
-                active = false;
-            }
+        } while (!__any_sync(0xffffffffu, done));
+        if (done) {
+            g.step_count[L.run] = rec.count;
+            g.ckpt_count[L.run] = L.save_idx;
+            lane_end<Cfg>(L, a, &bt);
+            active = false;
         }
     }
     totals_flush(&bt, a);

@@ -77,20 +77,21 @@ struct Controller {
         return accept ? gain : min_nan(gain, G(Cfg::CTL_SAFETY));
     }
     // Returns the controller status bits; updates dt, accept and history.
-    // ``ts``: the run's tolerance scale in the gain precision
-    static __device__ __forceinline__ int update(C& dt, const R* ynew, const R* y, const R* err, int niters,
+    // ``ts``: the run's tolerance scale in the gain precision; ``dt_g``: dt in
+    // the gain precision (which the loop has at hand)
+    static __device__ __forceinline__ int update(C& dt, G dt_g, const R* ynew, const R* y, const R* err, int niters,
                                                  bool truncated, bool& accept, State& st, G ts) {
         if constexpr (Cfg::CTRL == CTRL_FIXED) {
             accept = true;
             return SUCCESS;
         } else {
-            return update_with_norm(dt, error_norm2(ynew, y, err, ts), niters, truncated, accept, st);
+            return update_with_norm(dt, dt_g, error_norm2(ynew, y, err, ts), niters, truncated, accept, st);
         }
     }
     // The same decision from an error norm computed elsewhere (the
     // warp-per-system path reduces it over the lanes).
-    static __device__ __forceinline__ int update_with_norm(C& dt, C nrm2_c, int niters, bool truncated, bool& accept,
-                                                           State& st) {
+    static __device__ __forceinline__ int update_with_norm(C& dt, G dt_g, C nrm2_c, int niters, bool truncated,
+                                                           bool& accept, State& st) {
         if constexpr (Cfg::CTRL == CTRL_FIXED) {
             accept = true;
             return SUCCESS;
@@ -134,7 +135,7 @@ struct Controller {
                     // unless the Newton count lowered fac (a constant fold
                     // when the step reports no Newton iterations).
                     const G l2 = log2_t(nrm2);
-                    const G ldt = log2_t(G(current_dt));
+                    const G ldt = log2_t(dt_g);
                     const G lprev = pymax(st.h1, G(LOG2_1EM16));
                     const G lsf = safety < tmp ? G(0) : log2_t(safety / tmp);
                     const G x_basic = -expo * l2;
@@ -157,8 +158,10 @@ struct Controller {
             gain = finish_gain(gain, accept);
             const bool freeze = accept && truncated;
             const C dt_new_raw = current_dt * C(gain);
-            dt = freeze ? current_dt : clampv(dt_new_raw, C(Cfg::DT_MIN), C(Cfg::DT_MAX));
-            return (freeze || dt_new_raw > C(Cfg::DT_MIN)) ? SUCCESS : STEP_TOO_SMALL;
+            const bool above_min = dt_new_raw > C(Cfg::DT_MIN);   // false for a NaN
+            const C dt_new = above_min ? pymin(dt_new_raw, C(Cfg::DT_MAX)) : C(Cfg::DT_MIN);
+            dt = freeze ? current_dt : dt_new;
+            return (freeze || above_min) ? SUCCESS : STEP_TOO_SMALL;
         }
     }
 };

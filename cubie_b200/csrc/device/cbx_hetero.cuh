@@ -40,11 +40,13 @@ __device__ __forceinline__ void drain_family(const cbx_solve_args& a, unsigned l
             }
         }
         if (!__any_sync(0xffffffffu, active)) break;
-        if (active) {
-            if (lane_iterate<Cfg>(L, a)) {
-                lane_end<Cfg>(L, a, bt);
-                active = false;
-            }
+        bool done = false;
+        do {
+            if (active) done = lane_iterate<Cfg>(L, a);
+        } while (!__any_sync(0xffffffffu, done));
+        if (done) {
+            lane_end<Cfg>(L, a, bt);
+            active = false;
         }
     }
 }

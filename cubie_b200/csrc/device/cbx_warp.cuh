@@ -861,7 +861,7 @@ __device__ __forceinline__ bool warp_iterate(WarpLane<Cfg>& L, WarpCtx<Cfg>& w, 
         }
         nrm2 = warp_sum(nrm2) * C(Cfg::CTL_INV_N);
         bool ctl_accept = false;
-        const int ctl_status = Controller<Cfg>::update_with_norm(L.dt, nrm2, nit, truncated, ctl_accept, L.ctl);
+        const int ctl_status = Controller<Cfg>::update_with_norm(L.dt, G(L.dt), nrm2, nit, truncated, ctl_accept, L.ctl);
         accept = ctl_accept && !step_failed;
         L.iteration_status |= ctl_status;
         L.irrecoverable = L.irrecoverable || ((ctl_status & STEP_TOO_SMALL) != 0);
