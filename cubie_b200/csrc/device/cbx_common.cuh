@@ -108,6 +108,20 @@ __device__ __forceinline__ double log2_t(double a) { return log2(a); }
 __device__ __forceinline__ float exp2_t(float a) { return exp2f(a); }
 __device__ __forceinline__ double exp2_t(double a) { return exp2(a); }
 
+// c a^x b^y for a, b > 0.  In FP64 on the device one exponential serves both
+// powers (Tsit5 FP64, 50,021 Lorenz runs: 996 -> 942 us); in FP32 the two
+// approximate powers side by side have the shorter chain.
+__device__ __forceinline__ float scaled_powers(float c, float a, float x, float b, float y) {
+    return c * pow_t(a, x) * pow_t(b, y);
+}
+__device__ __forceinline__ double scaled_powers(double c, double a, double x, double b, double y) {
+#ifdef CBX_HOST_EMULATION
+    return c * pow_t(a, x) * pow_t(b, y);
+#else
+    return c * exp2(x * log2(a) + y * log2(b));
+#endif
+}
+
 template <class T> struct Limits;
 template <> struct Limits<float> {
     static __device__ __forceinline__ float huge() { return 3.4028234663852886e38f; }

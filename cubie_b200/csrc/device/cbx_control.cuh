@@ -108,10 +108,8 @@ struct Controller {
                 gain = G(safety * gpow(nrm2, -G(Cfg::CTL_E1)));
             } else if constexpr (Cfg::CTRL == CTRL_PI) {
                 const G err_prev = st.h0;
-                const G pgain = gpow(nrm2, -G(Cfg::CTL_E1));
                 const G src = err_prev > G(0) ? err_prev : nrm2;
-                const G igain = gpow(src, -G(Cfg::CTL_E2));
-                gain = safety * pgain * igain;
+                gain = scaled_powers(safety, nrm2, -G(Cfg::CTL_E1), src, -G(Cfg::CTL_E2));
                 st.h0 = commit_history ? nrm2 : err_prev;
             } else if constexpr (Cfg::CTRL == CTRL_PID) {
                 const G err_prev = st.h0, err_prev_prev = st.h1;
