@@ -74,12 +74,16 @@ def bytes_per_run(solver, prep, per_run_arrays: int = 0) -> int:
     """Device bytes one run needs: initial values, parameters, every output
     and ``per_run_arrays`` float64 per-run inputs (horizon, tolerance
     scale) plus the int64 claim order."""
+    known = prep.setdefault("bytes_per_run", {})
+    if per_run_arrays in known:
+        return known[per_run_arrays]
     itemsize = np.dtype(solver.precision).itemsize
     sysm = solver.system
     total = (sysm.num_states + max(sysm.num_parameters, 1)) * itemsize
     total += 8 * per_run_arrays + (8 if per_run_arrays else 0)
     for shape, dt in output_shapes(solver, prep, 1).values():
         total += int(np.prod(shape)) * np.dtype(dt).itemsize
+    known[per_run_arrays] = total
     return total
 
 

@@ -117,18 +117,19 @@ class HeteroSolver:
         return fams, routes
 
     def _module(self, preps):
-        fams = []
-        for s, prep in zip(self.solvers, preps):
-            fams.append((s.system, prep["spec"], prep["gen"].system))
-        src = generate_hetero_kernel(fams)
-        import hashlib
-        key = (hashlib.sha256(src.encode()).hexdigest(), self.device)
+        # each family's own kernel source fixes its part of the module (the
+        # block size is the launch's), so a known combination is found without
+        # generating the joint source again
+        first = self.solvers[0]
+        key = (tuple(prep["gen"].key for prep in preps), int(first.block_size), bool(first.fast_math), self.device)
         mod = _HETERO_MODULES.get(key)
         if mod is None:
-            cubin, log = _native.compile_cubin(src, _native.default_options(fast_math=self.solvers[0].fast_math))
+            src = generate_hetero_kernel([(s.system, prep["spec"], prep["gen"].system)
+                                          for s, prep in zip(self.solvers, preps)])
+            cubin, log = _native.compile_cubin(src, _native.default_options(fast_math=first.fast_math))
             mod = _native.Module(cubin, self.device, log)
             _HETERO_MODULES[key] = mod
-        return mod, src
+        return mod
 
     def setup(self, batches: Sequence[Dict[str, Any]]) -> "HeteroLaunch":
         """Allocate the outputs and build the launch arguments for
@@ -174,7 +175,7 @@ class HeteroSolver:
             args.append(a)
             keep += [it, pt, dt, tt]
             first.append(first[-1] + n)
-        mod, _ = self._module(preps)
+        mod = self._module(preps)
         h = _native.HeteroArgs()
         for k, a in enumerate(args):
             h.family[k] = a

@@ -18,6 +18,7 @@ from __future__ import annotations
 
 import hashlib
 from dataclasses import dataclass, field, replace
+from functools import cached_property
 from typing import Dict, List, Optional, Sequence, Tuple
 
 import numpy as np
@@ -208,7 +209,7 @@ class GeneratedKernel:
     system: GeneratedSystem
     spec: KernelSpec
 
-    @property
+    @cached_property
     def key(self) -> str:
         return hashlib.sha256(self.source.encode()).hexdigest()[:24]
 

@@ -64,6 +64,10 @@ IGNORED_KEYS = {"memory_settings", "cache", "auto_memory", "lineinfo", "time_log
 RENAMED = {"dt_save": "save_every", "dt_summarise": "summarise_every",
            "dt_update_summaries": "sample_summaries_every"}
 
+# prepared launches (kernel source, module, output sizes) a solver keeps, the
+# oldest dropped first
+PREPARED_MAX = 64
+
 _MODULE_CACHE: Dict[Tuple[str, int], "_native.Module"] = {}
 
 
@@ -582,16 +586,18 @@ class Solver:
         sizes for a launch."""
         if duration <= 0:
             raise ValueError("duration must be positive")
-        key = None
-        if interp is None:
-            key = (float(duration), float(settling_time), float(t0), durations is None, bool(load))
-            hit = self.__dict__.setdefault("_prepared", {}).get(key)
-            if hit is not None:
-                return hit
+        # driven systems differ by their driver table's shape, which is compiled in
+        driver_meta = interp.device_meta() if interp is not None else None
+        key = (float(duration), float(settling_time), float(t0), durations is None, bool(load),
+               None if driver_meta is None else tuple(sorted(driver_meta.items())), self.block_size,
+               self.min_blocks_per_sm, self.scratch_placement, self.max_registers)
+        prepared = self.__dict__.setdefault("_prepared", {})
+        hit = prepared.get(key)
+        if hit is not None:
+            return hit
         timing = self._timing(float(duration))
         if durations is not None and (timing["save_regularly"] or timing["summarise_regularly"]):
             raise ValueError("per-run durations need end-of-run saving only (no save_every or summaries)")
-        driver_meta = interp.device_meta() if interp is not None else None
         spec = self.kernel_spec(timing, driver_meta)
         if load:
             mod, gk = self.module_for(spec)
@@ -605,8 +611,9 @@ class Solver:
         summ_stop = summary_stop_time(duration, settling_time, t0, timing["sample_every"], p)
         prep = dict(timing=timing, spec=spec, module=mod, gen=gk, n_save=n_save, n_summ=n_summ,
                     save_stop=save_stop, summary_stop=summ_stop)
-        if key is not None:
-            self._prepared[key] = prep
+        while len(prepared) >= PREPARED_MAX:
+            prepared.pop(next(iter(prepared)), None)
+        prepared[key] = prep
         return prep
 
     def run(self, inits: np.ndarray, params: np.ndarray, interp=None, duration: float = 1.0,
@@ -677,7 +684,7 @@ class Solver:
             coeff_t = torch.as_tensor(interp.coefficients.astype(self.precision), device=dev).contiguous()
         order_t = self.run_order(dur_t, tol_t)
         args = self.make_args(prep, bufs, inits_t, params_t, coeff_t, n_runs, duration, settling_time, t0,
-                              dur_t, tol_t, order_t=order_t)
+                              dur_t, tol_t, order_t=order_t, zero_work=False)   # fresh buffers
         kernel = self.launch_kind
         s = stream if stream is not None else torch.cuda.current_stream(dev)
         e0 = torch.cuda.Event(enable_timing=True)
@@ -717,10 +724,13 @@ class Solver:
             "obs_sum": torch.zeros((n_summ, len(spec.summarised_observable_indices) * per_var, n_runs), device=dev,
                                    dtype=tdtype) if spec.summarised_observable_indices and per_var else None,
             "counters": torch.zeros((n_save, 4, n_runs), device=dev, dtype=torch.int32) if spec.save_counters else None,
-            "status": torch.zeros((n_runs,), device=dev, dtype=torch.int32),
-            "work": torch.zeros((2,), device=dev, dtype=torch.int64),
-            "totals": torch.zeros((4,), device=dev, dtype=torch.int64),
         }
+        # the small buffers share one allocation: cleared in one launch and
+        # read back in one copy (a fill or a copy of a few bytes costs as much
+        # as one of a megabyte)
+        small = torch.zeros((6 + (n_runs + 1) // 2,), device=dev, dtype=torch.int64)
+        bufs["work"], bufs["totals"] = small[:2], small[2:6]
+        bufs["status"] = small[6:].view(torch.int32)[:n_runs]
         return bufs
 
     def run_order(self, dur_t, tol_t=None):
@@ -759,7 +769,7 @@ class Solver:
 
     def make_args(self, prep, bufs, inits_t, params_t, coeff_t, n_runs, duration, settling_time, t0,
                   dur_t=None, tol_t=None, max_steps=None, order_t=None,
-                  run_stride=None) -> "_native.SolveArgs":
+                  run_stride=None, zero_work=True) -> "_native.SolveArgs":
         def ptr(t):
             return t.data_ptr() if t is not None else None
         a = _native.SolveArgs()
@@ -774,7 +784,8 @@ class Solver:
         a.status_out = ptr(bufs["status"])
         a.durations = ptr(dur_t)
         a.tol_scale = ptr(tol_t)
-        bufs["work"].zero_()
+        if zero_work:
+            bufs["work"].zero_()
         a.work_counter = ptr(bufs["work"])
         a.totals = ptr(bufs["totals"])
         a.abort_flag = None
@@ -809,11 +820,18 @@ class Solver:
             # buffer one output at a time
             torch = _torch()
             pinned = {}
+            together = bufs["status"].data_ptr() == bufs["totals"].data_ptr() + 32   # as allocate_outputs lays them
             for key in keys:
                 t = bufs.get(key)
-                if t is not None:
+                if t is not None and not (together and key in ("status", "totals")):
                     pinned[key] = torch.empty(tuple(t.shape), dtype=t.dtype, pin_memory=True)
                     pinned[key].copy_(t, non_blocking=True)
+            if together:
+                words = 4 + (n_runs + 1) // 2
+                small = torch.empty((words,), dtype=torch.int64, pin_memory=True)
+                small.copy_(bufs["totals"].as_strided((words,), (1,)), non_blocking=True)
+                pinned["totals"] = small[:4]
+                pinned["status"] = small[4:].view(torch.int32)[:n_runs]
             torch.cuda.current_stream(bufs["status"].device).synchronize()
             out = {k: (pinned[k].numpy() if k in pinned else None) for k in keys}
         res = SolveResult(
