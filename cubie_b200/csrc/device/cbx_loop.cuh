@@ -443,6 +443,17 @@ __device__ __forceinline__ long long claim_run(unsigned long long* counter) {
     return (long long)(base + rank);
 }
 
+// Whether the calling lane takes runs: with fewer runs than lanes each warp
+// uses only as many lanes as spread the runs evenly over the grid's warps.
+__device__ __forceinline__ bool lane_in_use(long long n_runs) {
+#ifdef CBX_HOST_EMULATION
+    return true;
+#else
+    const long long warps = (long long)gridDim.x * (blockDim.x >> 5);
+    return (long long)(threadIdx.x & 31) * warps < n_runs;
+#endif
+}
+
 // Persistent work-stealing kernel: resident warps loop until the run
 // counter is exhausted; a lane whose run finishes claims a new one at the
 // top of the next iteration.  Claims follow ``run_order`` when given (the
@@ -454,7 +465,7 @@ __device__ __forceinline__ void run_persistent(const cbx_solve_args a) {
     __shared__ BlockTotals bt;
     totals_begin(&bt);
     Lane<Cfg> L;
-    bool active = false, exhausted = false;
+    bool active = false, exhausted = !lane_in_use(a.n_runs);
     while (true) {
         if (!active && !exhausted) {
             const long long k = claim_run(a.work_counter);

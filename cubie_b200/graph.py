@@ -54,9 +54,7 @@ class GraphSolve:
             sms = _native.device_info(solver.device)["sm_count"]
             self.grid = max(1, min(max(per_sm, 1) * sms, (self.n_runs + self.block // 32 - 1) // (self.block // 32)))
         elif self.kernel == 1:
-            per_sm = prep["module"].occupancy(1, self.block)
-            sms = _native.device_info(solver.device)["sm_count"]
-            self.grid = max(1, min(max(per_sm, 1) * sms, (self.n_runs + self.block - 1) // self.block))
+            self.grid = 0      # the library's choice, fixed by the capture
         else:
             self.grid = (self.n_runs + self.block - 1) // self.block
         # pinned host staging and device buffers
