@@ -824,7 +824,7 @@ __device__ __forceinline__ void run_adjoint_forward_records(const cbx_solve_args
     __shared__ BlockTotals bt;
     totals_begin(&bt);
     Lane<Cfg> L;
-    bool active = false, exhausted = false;
+    bool active = false, exhausted = !lane_in_use(a.n_runs);
     const int cap = g.max_ckpts * g.ckpt_every;
     const long long step_step = g.lane_words * SegRecord<Cfg>::F;   // values from a run's record to its next
     RecordWriter<Cfg> rec{nullptr, step_step, 0};
@@ -881,7 +881,7 @@ __device__ __forceinline__ void run_adjoint_backward_records(const cbx_solve_arg
     long long run = -1;
     const R* rec_at = nullptr;   // the record in ``nxt``
     int j = -1, rows_end = 0;
-    bool active = false, exhausted = false;
+    bool active = false, exhausted = !lane_in_use(a.n_runs);
     while (true) {
         if (!active && !exhausted) {
             run = claim_run(a.work_counter);
