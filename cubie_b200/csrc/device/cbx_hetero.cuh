@@ -99,10 +99,16 @@ struct FamilyCount {
 
 }  // namespace cbx
 
+// Launch bounds: the block size, plus a minimum of resident blocks where the
+// generator asks for one (kernelgen.generate_hetero_kernel).
+#ifndef CBX_HETERO_BOUNDS
+#define CBX_HETERO_BOUNDS(BLOCK) __launch_bounds__(BLOCK)
+#endif
+
 // The size of cbx_hetero_probe tells the host how many families the
 // module was generated for.
 #define CBX_DEFINE_HETERO_KERNEL(BLOCK, ...)                                                          \
     __constant__ char cbx_hetero_probe[cbx::FamilyCount<__VA_ARGS__>::value];                         \
-    extern "C" __global__ void __launch_bounds__(BLOCK) cbx_integrate_hetero(cbx_hetero_args h) {    \
+    extern "C" __global__ void CBX_HETERO_BOUNDS(BLOCK) cbx_integrate_hetero(cbx_hetero_args h) {    \
         cbx::run_hetero<__VA_ARGS__>(h);                                                              \
     }
