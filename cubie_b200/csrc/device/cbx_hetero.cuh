@@ -28,6 +28,7 @@ namespace cbx {
 template <class Cfg>
 __device__ __forceinline__ void drain_family(const cbx_solve_args& a, unsigned long long* counter, BlockTotals* bt) {
     Lane<Cfg> L{};
+    Pass<Cfg> pass{};
     bool active = false, exhausted = false;
     while (true) {
         if (!active && !exhausted) {
@@ -42,7 +43,7 @@ __device__ __forceinline__ void drain_family(const cbx_solve_args& a, unsigned l
         if (!__any_sync(0xffffffffu, active)) break;
         bool done = false;
         do {
-            if (active) done = lane_iterate<Cfg>(L, a);
+            if (active) done = pass.advance(L, a);
         } while (!__any_sync(0xffffffffu, done));
         if (done) {
             lane_end<Cfg>(L, a, bt);

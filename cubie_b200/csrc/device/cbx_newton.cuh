@@ -195,26 +195,37 @@ template <class P> struct HasFused<P, decltype(void(P::FUSED))> { static constex
 // ``Prob`` supplies: K, residual(u, out) (out = u - h f(...)),
 // linearize(u) (fixes the Jacobians for the linear solve), op(), and
 // corr_norm2(delta, u) (the correction norm).
+//
+// The state of a solve between its iterations, so that a loop over runs can
+// take one iteration at a time (``NewtonState``); ``newton_solve`` runs one
+// to its end.
 template <class Cfg, class Prob>
-__device__ __forceinline__ int newton_solve(Prob& prob, typename Cfg::R* u, typename Cfg::C& prev_theta_store,
-                                            int& newton_iters, int& krylov_iters) {
+struct NewtonState {
     using R = typename Cfg::R;
     using C = typename Cfg::C;
-    constexpr int K = Prob::K;
-    const C kappa = C(0.01);
-    const C first_bound = C(1.0e-5);
-    const C theta_decay = C(0.3);
-    const C theta_div = C(2.0);
-    const C stag_eps = C(100.0) * sqrt_t(C(Limits<R>::eps()));
-    const C huge = C(Limits<R>::huge());
-    C prev_theta = (prev_theta_store > C(0)) ? prev_theta_store : C(1);
-    C ndz_prev = C(0);
-    bool converged = false, failed = false;
-    int last_lin = SUCCESS;
-    int iters = 0, total_k = 0;
-    R res[K], delta[K];
-    for (int it = 0; it < Cfg::NEWTON_MAX_ITERS; ++it) {
-        if (converged || failed) break;
+    static constexpr int K = Prob::K;
+    C prev_theta, ndz_prev;
+    int last_lin, iters, total_k;
+    bool converged, failed;
+    __device__ __forceinline__ void begin(C theta_store) {
+        prev_theta = (theta_store > C(0)) ? theta_store : C(1);
+        ndz_prev = C(0);
+        last_lin = SUCCESS;
+        iters = total_k = 0;
+        converged = failed = false;
+    }
+    __device__ __forceinline__ bool over() const {
+        return converged || failed || iters >= Cfg::NEWTON_MAX_ITERS;
+    }
+    // One correction of ``u``.
+    __device__ __forceinline__ void iterate(Prob& prob, R* u) {
+        const C kappa = C(0.01);
+        const C first_bound = C(1.0e-5);
+        const C theta_decay = C(0.3);
+        const C theta_div = C(2.0);
+        const C stag_eps = C(100.0) * sqrt_t(C(Limits<R>::eps()));
+        const C huge = C(Limits<R>::huge());
+        R res[K], delta[K];
         if constexpr (HasFused<Prob>::value) prob.residual_linearize(u, res);
         else prob.residual(u, res);
 #pragma unroll
@@ -251,12 +262,23 @@ __device__ __forceinline__ int newton_solve(Prob& prob, typename Cfg::R* u, type
         ndz_prev = commit ? ndz : C(0);
         prev_theta = (judged && history) ? theta : prev_theta;
     }
-    prev_theta_store = converged ? prev_theta : C(1);
-    int fail_bits = failed ? NEWTON_DIVERGENCE : MAX_NEWTON_ITERATIONS_EXCEEDED;
-    if (last_lin != SUCCESS) fail_bits |= last_lin;
-    newton_iters = iters;
-    krylov_iters = total_k;
-    return converged ? SUCCESS : fail_bits;
+    __device__ __forceinline__ int end(C& theta_store) const {
+        theta_store = converged ? prev_theta : C(1);
+        int fail_bits = failed ? NEWTON_DIVERGENCE : MAX_NEWTON_ITERATIONS_EXCEEDED;
+        if (last_lin != SUCCESS) fail_bits |= last_lin;
+        return converged ? SUCCESS : fail_bits;
+    }
+};
+
+template <class Cfg, class Prob>
+__device__ __forceinline__ int newton_solve(Prob& prob, typename Cfg::R* u, typename Cfg::C& prev_theta_store,
+                                            int& newton_iters, int& krylov_iters) {
+    NewtonState<Cfg, Prob> st;
+    st.begin(prev_theta_store);
+    while (!st.over()) st.iterate(prob, u);
+    newton_iters = st.iters;
+    krylov_iters = st.total_k;
+    return st.end(prev_theta_store);
 }
 
 }  // namespace cbx

@@ -507,10 +507,15 @@ struct FirkStep {
             }
         }
     }
-    static __device__ __forceinline__ int step(const StepCtx<Cfg>& ctx, const R* y, R* ynew, R* delta, R* err,
-                                               const R*, R* drv_new, R dt, R t, bool first_step,
-                                               bool prev_accepted, Persist& ps, Iters& its) {
-        its = Iters{};
+    // A step in the three parts a run loop may take one at a time: the start
+    // (prediction, stage drivers), Newton iterations until ``newton.over()``,
+    // and the end.
+    struct Work {
+        R drv_stack[S][ND > 0 ? ND : 1];
+        NewtonState<Cfg, FirkProblem<Cfg>> newton;
+    };
+    static __device__ __forceinline__ void step_begin(const StepCtx<Cfg>& ctx, R dt, R t, bool first_step,
+                                                      bool prev_accepted, Persist& ps, Work& w) {
         if (Tab::DENSE_PRED) {
             const R previous_dt = ps.prev_dt;
             ps.prev_dt = dt;
@@ -519,18 +524,28 @@ struct FirkStep {
             const bool apply = !first_step && prev_accepted && (ratio <= R(Tab::PRED_RATIO_LIMIT));
             predict(ps.u, ratio, apply);
         }
-        R drv_stack[S][ND > 0 ? ND : 1];
         if constexpr (ND > 0) {
 #pragma unroll
-            for (int i = 0; i < S; ++i) Drivers<Cfg>::eval(t + dt * R(Tab::c(i)), ctx.coeffs, drv_stack[i]);
+            for (int i = 0; i < S; ++i) Drivers<Cfg>::eval(t + dt * R(Tab::c(i)), ctx.coeffs, w.drv_stack[i]);
         }
+        w.newton.begin(ps.theta);
+    }
+    static __device__ __forceinline__ void step_iterate(const StepCtx<Cfg>& ctx, const R* y, R dt, R t, Persist& ps,
+                                                        Work& w) {
         FirkProblem<Cfg> prob;
         prob.ctx = &ctx;
         prob.base = y;
-        prob.drv = drv_stack;
+        prob.drv = w.drv_stack;
         prob.t = t;
         prob.h = dt;
-        const int status = newton_solve<Cfg>(prob, ps.u, ps.theta, its.nit, its.kit);
+        w.newton.iterate(prob, ps.u);
+    }
+    static __device__ __forceinline__ int step_end(const StepCtx<Cfg>& ctx, const R* y, R* ynew, R* delta, R* err,
+                                                   R* drv_new, R dt, R t, Persist& ps, Work& w, Iters& its) {
+        its = Iters{};
+        const int status = w.newton.end(ps.theta);
+        its.nit = w.newton.iters;
+        its.kit = w.newton.total_k;
         its.nit_all = its.nit;
         its.kit_all = its.kit;
         if (!Tab::ACC_OUT) {
@@ -578,12 +593,20 @@ struct FirkStep {
         if constexpr (ND > 0) {
             if (Tab::c(S - 1) == 1.0) {
 #pragma unroll
-                for (int q = 0; q < ND; ++q) drv_new[q] = drv_stack[S - 1][q];
+                for (int q = 0; q < ND; ++q) drv_new[q] = w.drv_stack[S - 1][q];
             } else {
                 Drivers<Cfg>::eval(t + dt, ctx.coeffs, drv_new);
             }
         }
         return status;
+    }
+    static __device__ __forceinline__ int step(const StepCtx<Cfg>& ctx, const R* y, R* ynew, R* delta, R* err,
+                                               const R*, R* drv_new, R dt, R t, bool first_step,
+                                               bool prev_accepted, Persist& ps, Iters& its) {
+        Work w;
+        step_begin(ctx, dt, t, first_step, prev_accepted, ps, w);
+        while (!w.newton.over()) step_iterate(ctx, y, dt, t, ps, w);
+        return step_end(ctx, y, ynew, delta, err, drv_new, dt, t, ps, w, its);
     }
 };
 
