@@ -66,7 +66,7 @@ RENAMED = {"dt_save": "save_every", "dt_summarise": "summarise_every",
 
 # prepared launches (kernel source, module, output sizes) a solver keeps, the
 # oldest dropped first
-PREPARED_MAX = 64
+PREPARED_MAX = 512
 
 _MODULE_CACHE: Dict[Tuple[str, int], "_native.Module"] = {}
 
