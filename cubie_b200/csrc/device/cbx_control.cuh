@@ -56,7 +56,7 @@ struct Controller {
     static __device__ __forceinline__ G error_ratio(R e_i, R ynew_i, R y_i, G atol, G rtol, G ts) {
         const G e = max_nan(G(absv(e_i)), G(1e-16));
         const G tol = atol + rtol * ts * max_nan(G(absv(ynew_i)), G(absv(y_i)));
-        return e / tol;
+        return ratio_t(e, tol);
     }
     static __device__ __forceinline__ C error_norm2(const R* ynew, const R* y, const R* err, G ts) {
         C nrm2 = C(0);

@@ -35,7 +35,7 @@ __device__ __forceinline__ typename Cfg::C tol_ratio(typename Cfg::R v, typename
     } else {
         C tol = C(atol) + C(rtol) * scale * C(absv(ref));
         tol = max_nan(tol, C(1e-16));
-        return C(v) / tol;
+        return ratio_t(C(v), tol);
     }
 }
 
