@@ -116,8 +116,8 @@ __device__ __forceinline__ double exp2_t(double a) { return exp2(a); }
 // division's scaling and exceptional cases; within one unit in the last place
 // of the division (tests/test_ratio_gpu.py), an infinite quotient stays one.
 // Divisions were what the FP64 norms cost: Tsit5, 50,021 Lorenz runs 939 ->
-// 871 us; ROS3P, 20,001 Van der Pol runs 1.85 -> 1.60 ms; Radau IIA5 with
-// GMRES, 10,001 runs 7.04 -> 6.04 ms.
+// 884 us; ROS3P, 20,001 Van der Pol runs 1.85 -> 1.61 ms; Radau IIA5 with
+// GMRES, 10,001 runs 7.04 -> 6.09 ms.
 __device__ __forceinline__ float ratio_t(float e, float tol) { return e / tol; }
 __device__ __forceinline__ double ratio_t(double e, double tol) {
 #ifdef CBX_HOST_EMULATION
