@@ -68,7 +68,9 @@ RENAMED = {"dt_save": "save_every", "dt_summarise": "summarise_every",
 # oldest dropped first
 PREPARED_MAX = 512
 
-_MODULE_CACHE: Dict[Tuple[str, int], "_native.Module"] = {}
+# loaded modules by kernel source, compile options (fast math and register
+# caps are not in the source) and device
+_MODULE_CACHE: Dict[Tuple[str, Tuple[str, ...], int], "_native.Module"] = {}
 
 
 def _torch():
@@ -459,19 +461,23 @@ class Solver:
         several threads at once).  Returns ``(gk, cubin, log)``, or
         ``(gk, None, None)`` when the module is already loaded."""
         gk = self._generate(spec)
-        if (gk.key, self.device) in _MODULE_CACHE:
+        opts = self._compile_options(spec)
+        if (gk.key, opts, self.device) in _MODULE_CACHE:
             return gk, None, None
+        cubin, log = _native.compile_cubin(gk.source, opts)
+        return gk, cubin, log
+
+    def _compile_options(self, spec: KernelSpec) -> Tuple[str, ...]:
         opts = _native.default_options(fast_math=self.fast_math)
         if spec.max_registers:
             opts.append(f"--maxrregcount={int(spec.max_registers)}")
-        cubin, log = _native.compile_cubin(gk.source, opts)
-        return gk, cubin, log
+        return tuple(opts)
 
     def module_for(self, spec: KernelSpec, compiled=None):
         """Compile (or fetch) the NVRTC module for ``spec`` on this device;
         ``compiled`` is a result of :meth:`compile_for` to load instead."""
         gk, cubin, log = compiled if compiled is not None else self.compile_for(spec)
-        key = (gk.key, self.device)
+        key = (gk.key, self._compile_options(spec), self.device)
         mod = _MODULE_CACHE.get(key)
         if mod is None:
             if cubin is None:
