@@ -26,6 +26,7 @@ from __future__ import annotations
 
 import itertools
 import math
+import operator
 import time
 import warnings
 from dataclasses import replace
@@ -71,6 +72,19 @@ PREPARED_MAX = 512
 # loaded modules by kernel source, compile options (fast math and register
 # caps are not in the source) and device
 _MODULE_CACHE: Dict[Tuple[str, Tuple[str, ...], int], "_native.Module"] = {}
+
+
+# settings a launch's kernel, options and output sizes follow from (besides
+# the timing, the outputs and the tableau, which ``Solver._settings`` adds)
+_SCALAR_SETTINGS = operator.attrgetter(
+    "precision", "controller", "dt", "dt_min", "dt_max", "kp", "ki", "kd", "safety", "min_gain", "max_gain",
+    "deadband_min", "deadband_max", "newton_target_iters", "linear_correction_type", "krylov_max_iters",
+    "krylov_residual_reduction", "krylov_residual_floor", "newton_max_iters", "preconditioner_order",
+    "preconditioned", "gmres_restart", "mixed_precision", "block_size", "min_blocks_per_sm", "adjoint", "layout",
+    "attempt_dense_prediction", "scratch_placement", "max_registers", "fast_math", "device")
+_VECTOR_SETTINGS = operator.attrgetter("atol", "rtol", "krylov_atol", "krylov_rtol", "newton_atol", "newton_rtol")
+_LIST_SETTINGS = operator.attrgetter("saved_state_indices", "saved_observable_indices", "summarised_state_indices",
+                                     "summarised_observable_indices")
 
 
 def _torch():
@@ -586,6 +600,14 @@ class Solver:
                         durations=durations, tol_scale=tol_scale, stream=stream,
                         block=blocksize)
 
+    def _settings(self) -> Tuple:
+        """The settings of now, as a key: a prepared launch is used again
+        while they are the ones it was prepared under."""
+        return (_SCALAR_SETTINGS(self), id(self.tableau), tuple(self.flags.values()),
+                tuple(self._user_timing.values()), tuple(self.summary_plan.metrics),
+                *(tuple(v) for v in _LIST_SETTINGS(self)),
+                *(np.asarray(v, dtype=np.float64).tobytes() for v in _VECTOR_SETTINGS(self)))
+
     def prepare(self, duration: float, settling_time: float = 0.0, t0: float = 0.0,
                 interp=None, durations=None, load: bool = True) -> Dict[str, Any]:
         """Compile (and with ``load``, load) the module and compute output
@@ -595,8 +617,7 @@ class Solver:
         # driven systems differ by their driver table's shape, which is compiled in
         driver_meta = interp.device_meta() if interp is not None else None
         key = (float(duration), float(settling_time), float(t0), durations is None, bool(load),
-               None if driver_meta is None else tuple(sorted(driver_meta.items())), self.block_size,
-               self.min_blocks_per_sm, self.scratch_placement, self.max_registers)
+               None if driver_meta is None else tuple(sorted(driver_meta.items())), self._settings())
         prepared = self.__dict__.setdefault("_prepared", {})
         hit = prepared.get(key)
         if hit is not None:
