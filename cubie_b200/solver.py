@@ -638,8 +638,9 @@ class Solver:
         summ_stop = summary_stop_time(duration, settling_time, t0, timing["sample_every"], p)
         prep = dict(timing=timing, spec=spec, module=mod, gen=gk, n_save=n_save, n_summ=n_summ,
                     save_stop=save_stop, summary_stop=summ_stop)
-        while len(prepared) >= PREPARED_MAX:
-            prepared.pop(next(iter(prepared)), None)
+        # other threads may be preparing too: a snapshot of the keys, no iteration
+        for old in list(prepared)[:max(0, len(prepared) - PREPARED_MAX + 1)]:
+            prepared.pop(old, None)
         prepared[key] = prep
         return prep
 

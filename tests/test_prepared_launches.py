@@ -45,3 +45,43 @@ def test_changed_settings_are_prepared_anew(driven, change, source):
     else:
         assert after["n_save"] != before["n_save"]
     assert s.prepare(2.0, interp=interp, load=False) is after
+
+
+def test_threads_prepare_at_the_limit(monkeypatch):
+    """Several threads at a full table: the oldest entries go, nothing raises."""
+    import sys
+    import threading
+    from cubie_b200 import solver as solver_module
+    s = _solver()
+    interp = _interp(s)
+    one = s.prepare(1.0, interp=interp, load=False)
+    monkeypatch.setattr(solver_module, "PREPARED_MAX", 4)
+    # the preparation itself takes milliseconds: without it the threads meet
+    # at the table
+    monkeypatch.setattr(s, "_generate", lambda spec: one["gen"])
+    monkeypatch.setattr(s, "kernel_spec", lambda timing, meta=None: one["spec"])
+    errors = []
+    start = threading.Barrier(6)
+
+    def work(k):
+        start.wait()
+        try:
+            for i in range(400):
+                s.prepare(1.0 + k + 1e-3 * i, interp=interp, load=False)
+        except Exception as exc:
+            errors.append(exc)
+
+    interval = sys.getswitchinterval()
+    sys.setswitchinterval(1e-6)
+    try:
+        threads = [threading.Thread(target=work, args=(k,)) for k in range(6)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+    finally:
+        sys.setswitchinterval(interval)
+    assert not errors
+    assert len(s._prepared) <= 4 + 6
+    s.prepare(99.0, interp=interp, load=False)
+    assert len(s._prepared) <= 4
