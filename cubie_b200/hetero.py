@@ -52,6 +52,17 @@ def _take(x, idx):
     return np.asarray(x)[..., idx]
 
 
+def _per_run(values, n: int, name: str, dev):
+    """``values`` as one FP64 entry per run on ``dev`` (None stays None)."""
+    if values is None:
+        return None
+    torch = _torch()
+    t = torch.as_tensor(values).to(device=dev, dtype=torch.float64).reshape(-1).contiguous()
+    if t.numel() != n:
+        raise ValueError(f"{name} must have one entry per run")
+    return t
+
+
 class HeteroSolver:
     """One launch over the runs of several solvers.
 
@@ -162,9 +173,8 @@ class HeteroSolver:
             if pt.numel() == 0:
                 pt = torch.zeros((1, max(n, 1)), device=dev, dtype=tdt)
             bf = s.allocate_outputs(prep, n, dev, tdt)
-            dt = None if durs is None else torch.as_tensor(durs).to(device=dev, dtype=torch.float64).contiguous()
-            ts = b.get("tol_scale")
-            tt = None if ts is None else torch.as_tensor(ts).to(device=dev, dtype=torch.float64).contiguous()
+            dt = _per_run(durs, n, "durations", dev)
+            tt = _per_run(b.get("tol_scale"), n, "tol_scale", dev)
             # runs claimed by decreasing estimated work within each family
             order = s.run_order(dt, tt) if dt is not None else None
             a = s.make_args(prep, bf, it, pt, None, n, duration, b.get("settling_time", 0.0), b.get("t0", 0.0),

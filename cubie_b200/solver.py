@@ -761,6 +761,22 @@ class Solver:
         bufs["status"] = small[6:].view(torch.int32)[:n_runs]
         return bufs
 
+    @staticmethod
+    def _claim_work(dur_t, tol_t=None):
+        """(horizons, tolerance scales or None) as ``cbx_claim_order`` reads
+        them: FP64, contiguous, one entry per run each, on one device (a
+        single scale serves every run).  None for what it cannot read; the
+        general path then orders it or raises."""
+        torch = _torch()
+        n = int(dur_t.numel())
+        if dur_t.dtype != torch.float64 or dur_t.dim() != 1 or not dur_t.is_contiguous() or not 0 < n < 2 ** 32:
+            return None
+        if tol_t is None:
+            return dur_t, None
+        if tol_t.device != dur_t.device or tuple(tol_t.shape) not in ((n,), (1,), ()):
+            return None
+        return dur_t, tol_t.to(torch.float64).expand(n).contiguous()
+
     def run_order(self, dur_t, tol_t=None):
         """Claim order of a persistent launch: with per-run horizons and
         ``schedule='longest_first'`` (the default ``'auto'`` when horizons
@@ -779,14 +795,14 @@ class Solver:
         torch = _torch()
         scaled = tol_t is not None and self.controller != "fixed"
         q = max(int(getattr(self.tableau, "order", 1) or 1), 1)
-        n = int(dur_t.numel())
-        if dur_t.is_cuda and dur_t.dtype == torch.float64 and dur_t.dim() == 1 and dur_t.is_contiguous() \
-                and 0 < n < 2 ** 32:
+        work = self._claim_work(dur_t, tol_t if scaled else None) if dur_t.is_cuda else None
+        if work is not None:
+            n = int(dur_t.numel())
             order = torch.empty((n,), device=dur_t.device, dtype=torch.int64)
             scratch = torch.empty((_native.CLAIM_ORDER_SCRATCH_BYTES // 4,), device=dur_t.device, dtype=torch.int32)
-            scale = tol_t.to(torch.float64).reshape(-1).contiguous() if scaled else None
+            horizon, scale = work
             with torch.cuda.device(dur_t.device):
-                _native.claim_order(dur_t.data_ptr(), None if scale is None else scale.data_ptr(), -1.0 / (q + 1), n,
+                _native.claim_order(horizon.data_ptr(), None if scale is None else scale.data_ptr(), -1.0 / (q + 1), n,
                                     order.data_ptr(), scratch.data_ptr(),
                                     torch.cuda.current_stream(dur_t.device).cuda_stream)
             return order
