@@ -1018,7 +1018,8 @@ def main():
     ap.add_argument("--cpu-max-steps", type=int, default=3000)
     ap.add_argument("--no-cpu", action="store_true")
     ap.add_argument("--block", type=int, default=128, help="block size of the headline launches")
-    ap.add_argument("--min-blocks", type=int, default=1, help="minimum resident blocks per SM (register cap)")
+    ap.add_argument("--min-blocks", type=int, default=0,
+                    help="minimum resident blocks per SM (register cap; 0: the library's rule, 1: none)")
     ap.add_argument("--headline-only", action="store_true",
                     help="time the headline launch only and print its record (for profiling)")
     ap.add_argument("--ref-per-core", type=int, default=1, help="--impl reference: runs per core per pass")

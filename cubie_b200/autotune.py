@@ -31,8 +31,14 @@ from typing import Callable, Dict, Iterable, List, Optional, Sequence, Tuple
 
 import numpy as np
 
+from .kernelgen import bounds_registers
+
+# (block size, minimum of resident blocks per SM: 1 for none, 0 for the kernel
+# generator's rule)
 DEFAULT_CANDIDATES: Tuple[Tuple[int, int], ...] = ((128, 1), (64, 1), (256, 1), (32, 1), (128, 4), (128, 6),
                                                     (64, 8), (256, 2))
+# tried first where the rule asks for more than none
+RULE_CANDIDATES: Tuple[Tuple[int, int], ...] = ((128, 0), (64, 0), (32, 0))
 
 
 # warp-per-system layout: fewer shapes (each compile of a large system is
@@ -40,8 +46,8 @@ DEFAULT_CANDIDATES: Tuple[Tuple[int, int], ...] = ((128, 1), (64, 1), (256, 1), 
 # the placements that pass vectors by address (with "registers" the call
 # keeps them live and the compiler takes what it needs)
 WARP_CANDIDATES: Tuple[Tuple[int, int, str, int], ...] = tuple(
-    (b, 1, p, r) for b in (128, 64) for p in ("shared", "local") for r in (0, 168)) + tuple(
-    (b, 1, "registers", 0) for b in (128, 64))
+    (b, 0, p, r) for b in (128, 64) for p in ("shared", "local") for r in (0, 168)) + tuple(
+    (b, 0, "registers", 0) for b in (128, 64)) + tuple((128, 1, p, 0) for p in ("local", "registers"))
 
 
 # runs of the caller's batch timed per candidate
@@ -52,7 +58,10 @@ def default_candidates(solver) -> List[Tuple]:
     if solver.layout == "warp":
         if getattr(solver, "placement_pending", False):
             return list(WARP_CANDIDATES)
-        return [(b, 1, solver.scratch_placement, r) for b in (128, 64) for r in (0, 168)]
+        return [(b, 0, solver.scratch_placement, r) for b in (128, 64) for r in (0, 168)] + [
+            (128, 1, solver.scratch_placement, 0)]
+    if bounds_registers(solver.tableau.kind, solver.linear_correction_type):
+        return [*RULE_CANDIDATES, *DEFAULT_CANDIDATES]
     return list(DEFAULT_CANDIDATES)
 
 

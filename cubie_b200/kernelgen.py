@@ -97,7 +97,9 @@ class KernelSpec:
     # execution policy
     mixed_precision: bool = False
     block_size: int = 128
-    min_blocks_per_sm: int = 1
+    # minimum of resident blocks per SM asked of the compiler (0: the rules of
+    # ``thread_min_blocks`` and ``warp_min_blocks``; 1: none)
+    min_blocks_per_sm: int = 0
     dense_prediction: Optional[bool] = None
     # discrete adjoint kernels (forward with checkpoints, reverse sweep)
     adjoint: bool = False
@@ -366,10 +368,16 @@ def family_block(system: SymbolicODE, spec: KernelSpec, gen: GeneratedSystem, ns
     return lines
 
 
+def bounds_registers(kind: str, linear_correction_type: str) -> bool:
+    """Whether ``thread_min_blocks`` bounds the step's registers."""
+    return kind == FIRK or (kind == ROSENBROCK and linear_correction_type == "direct")
+
+
 def thread_min_blocks(spec: KernelSpec) -> int:
     """Minimum of resident blocks per SM in the kernels' launch bounds (0:
-    none): the caller's, or where none was asked for 256 threads' worth for
-    fully implicit steps and direct Rosenbrock steps.
+    none): the caller's, or where the caller named neither it nor a register
+    cap, 256 threads' worth for fully implicit steps and direct Rosenbrock
+    steps.
 
     Without one the compiler holds these kernels to the registers of a higher
     occupancy than they profit from; asked for two 128-thread blocks it spends
@@ -379,10 +387,11 @@ def thread_min_blocks(spec: KernelSpec) -> int:
     with FP64 control, 524,288 runs 2.70 -> 2.65.  Explicit steps and Rosenbrock
     or DIRK steps with a Krylov solver lose or stay (Tsit5 FP64 2.19 -> 2.30,
     ROS3P with GMRES 4.31 -> 4.44, SDIRK4 0.98 -> 0.99); more blocks spill."""
-    if int(spec.min_blocks_per_sm) > 1:
-        return int(spec.min_blocks_per_sm)
-    kind = spec.tableau.kind
-    if kind == FIRK or (kind == ROSENBROCK and spec.linear_correction_type == "direct"):
+    if int(spec.min_blocks_per_sm):
+        return int(spec.min_blocks_per_sm) if int(spec.min_blocks_per_sm) > 1 else 0
+    if spec.max_registers:
+        return 0
+    if bounds_registers(spec.tableau.kind, spec.linear_correction_type):
         return max(1, 256 // int(spec.block_size))
     return 0
 
@@ -430,7 +439,7 @@ def generate_hetero_kernel(families: Sequence[Tuple[SymbolicODE, KernelSpec, Gen
     # the register allowance of the family that profits from one (Lorenz
     # DP54, Van der Pol and Robertson under direct ROS3P, 50,000 runs each:
     # 2.09 -> 1.90 ms)
-    min_blocks = max(thread_min_blocks(replace(spec, block_size=block, min_blocks_per_sm=1))
+    min_blocks = max(thread_min_blocks(replace(spec, block_size=block, min_blocks_per_sm=0, max_registers=0))
                      for _, spec, _ in families)
     if min_blocks:
         lines.append(f"#define CBX_HETERO_BOUNDS(BLOCK) __launch_bounds__(BLOCK, {min_blocks})")
@@ -449,7 +458,7 @@ def generate_hetero_kernel(families: Sequence[Tuple[SymbolicODE, KernelSpec, Gen
 
 def warp_min_blocks(spec: KernelSpec, warp_code) -> int:
     """Minimum of resident blocks per SM asked for the warp kernel's register
-    form (0: the compiler's own choice).
+    form (0: the compiler's own choice); a caller's own goes first.
 
     Left to itself the compiler gave the 256-state cable 168 or 212 registers
     (12 or 8 resident warps; 1.33 or 1.79 ms) from one small change of the
@@ -460,6 +469,8 @@ def warp_min_blocks(spec: KernelSpec, warp_code) -> int:
     2.03 / 2.50, 384 1.37 / 1.96 / 2.60, 512 2.03 / 2.93 / 3.94: 16 warps
     where the lane's vectors then just fit 128 registers, 12 where they fit
     168, and no bound where it would spill them or is not needed."""
+    if int(spec.min_blocks_per_sm):
+        return int(spec.min_blocks_per_sm) if int(spec.min_blocks_per_sm) > 1 else 0
     if not warp_code.register_slots or spec.max_registers:
         return 0
     nbytes = np.dtype(spec.precision).itemsize * (10 * warp_code.register_slots + warp_code.register_coefs)

@@ -157,7 +157,8 @@ class Solver:
         bs = execution.get("block_size", 128)
         self.autotune_pending = isinstance(bs, str) and bs == "auto"
         self.block_size = 128 if self.autotune_pending else int(bs)
-        self.min_blocks_per_sm = int(execution.get("min_blocks_per_sm", 1))
+        # minimum of resident blocks per SM (0: the kernel generator's rules, 1: none)
+        self.min_blocks_per_sm = int(execution.get("min_blocks_per_sm", 0))
         self.adjoint = bool(execution.get("adjoint", False))
         # "thread": one run per thread; "warp": one run per warp, for large
         # systems (diagonally implicit tableaus); "auto": warp from 64 states
