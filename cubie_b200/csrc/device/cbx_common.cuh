@@ -108,27 +108,30 @@ __device__ __forceinline__ double log2_t(double a) { return log2(a); }
 __device__ __forceinline__ float exp2_t(float a) { return exp2f(a); }
 __device__ __forceinline__ double exp2_t(double a) { return exp2(a); }
 
-// e / tol for a positive tolerance in the normal range (the norms' weights:
-// 1e-16 up to rtol times the state).  In FP64 on the device: the hardware's
-// approximate reciprocal refined by two Newton iterations, then the quotient
-// corrected by its residual (Markstein, Computation of elementary functions on
-// the IBM RISC System/6000, IBM J. Res. Dev. 34, 1990), without the general
-// division's scaling and exceptional cases; within one unit in the last place
-// of the division (tests/test_ratio_gpu.py), an infinite quotient stays one.
-// Divisions were what the FP64 norms cost: Tsit5, 50,021 Lorenz runs 939 ->
-// 884 us; ROS3P, 20,001 Van der Pol runs 1.85 -> 1.61 ms; Radau IIA5 with
-// GMRES, 10,001 runs 7.04 -> 6.09 ms.
+// e / tol of the norms.  In FP64 on the device: the hardware's approximate
+// reciprocal refined by two Newton iterations, then the quotient corrected by
+// its residual (Markstein, Computation of elementary functions on the IBM RISC
+// System/6000, IBM J. Res. Dev. 34, 1990), without the general division's
+// scaling; where that leaves the finite numbers (a zero or infinite tolerance,
+// an infinite or NaN term, an overflow) the product with the unrefined
+// reciprocal is the division's value.  For every term and tolerance of the
+// norms it has the division's bits (tests/test_ratio_gpu.py); tolerances below
+// 2^-1022 count as zero and those above 2^1021 as infinite.  Divisions were
+// what the FP64 norms cost: Tsit5, 50,021 Lorenz runs 939 -> 884 us; ROS3P,
+// 20,001 Van der Pol runs 1.85 -> 1.61 ms; Radau IIA5 with GMRES, 10,001 runs
+// 7.04 -> 6.09 ms.
 __device__ __forceinline__ float ratio_t(float e, float tol) { return e / tol; }
 __device__ __forceinline__ double ratio_t(double e, double tol) {
 #ifdef CBX_HOST_EMULATION
     return e / tol;
 #else
-    double r;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(tol));
-    r = fma(r, fma(-tol, r, 1.0), r);
+    double r0;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r0) : "d"(tol));
+    double r = fma(r0, fma(-tol, r0, 1.0), r0);
     r = fma(r, fma(-tol, r, 1.0), r);
     const double q = e * r;
-    return is_finite(q) ? fma(r, fma(-tol, q, e), q) : q;
+    const double corrected = fma(r, fma(-tol, q, e), q);
+    return is_finite(corrected) ? corrected : e * r0;
 #endif
 }
 
