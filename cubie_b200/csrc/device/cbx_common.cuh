@@ -93,16 +93,6 @@ __device__ __forceinline__ bool is_nan(double v) { return isnan(v); }
 __device__ __forceinline__ float sqrt_t(float v) { return sqrtf(v); }
 __device__ __forceinline__ double sqrt_t(double v) { return sqrt(v); }
 __device__ __forceinline__ float pow_t(float a, float b) { return powf(a, b); }
-#ifdef CBX_HOST_EMULATION
-__device__ __forceinline__ double pow_t(double a, double b) { return pow(a, b); }
-#else
-// a > 0 and |b log2 a| of a few units (error norms and step ratios under the
-// controllers' exponents): a few roundings at about half the instructions of
-// pow, which carries its logarithm to twice the precision.  The two powers of
-// a PI step were a fifth of an FP64 step's issue slots: Tsit5 on 50,021 Lorenz
-// runs 1.24 -> 1.03 ms, ROS3P on 20,001 Van der Pol runs 2.36 -> 1.89.
-__device__ __forceinline__ double pow_t(double a, double b) { return exp2(b * log2(a)); }
-#endif
 __device__ __forceinline__ float log2_t(float a) { return log2f(a); }
 __device__ __forceinline__ double log2_t(double a) { return log2(a); }
 __device__ __forceinline__ float exp2_t(float a) { return exp2f(a); }
@@ -135,6 +125,47 @@ __device__ __forceinline__ double ratio_t(double e, double tol) {
 #endif
 }
 
+#ifdef CBX_HOST_EMULATION
+__device__ __forceinline__ double pow_t(double a, double b) { return pow(a, b); }
+#else
+// The FP64 controllers' powers of error norms and step ratios.  pow carries
+// its logarithm to twice the precision, because log2 a has its exponent's
+// size and b log2 a loses that many bits to it.  Here a = 2^k m with m in
+// [1, 2): b k is formed exactly for b rounded to a multiple of 2^-40, its
+// integer part becomes the result's exponent, and log2 m, the remainder of b
+// and the fraction are a few units at most, so the result is about as close as
+// pow's (tests/test_gain_powers_gpu.py) at half its instructions.  Finite
+// a >= 0 (the controllers map other norms to 1e16); zero and subnormal a count
+// as 2^-1023 and infinity as 2^1024, whose powers lie beyond a gain's clamp.
+struct Log2Parts {
+    double k, m;      // a = 2^k 2^m, 0 <= m <= 1
+    __device__ __forceinline__ explicit Log2Parts(double a) {
+        const int hi = __double2hiint(a);
+        k = double((hi >> 20) - 1023);
+        m = log2(__hiloint2double((hi & 0x000fffff) | 0x3ff00000, __double2loint(a)));
+    }
+};
+// b to a multiple of 2^-40 (its product with an exponent is exact)
+__device__ __forceinline__ double coarse(double b) { return (b + 0x1.8p12) - 0x1.8p12; }
+// c 2^(whole + rest): ``whole`` a multiple of 2^-40, ``rest`` a few units.  What
+// their sum's rounding loses multiplies the result.
+__device__ __forceinline__ double scaled_exp2(double c, double whole, double rest) {
+    const double shifted = whole + 0x1.8p52;               // rounds to an integer
+    const double fraction = whole - (shifted - 0x1.8p52);
+    const double f = fraction + rest;
+    const double lost = (fraction - f) + rest;
+    int n = __double2loint(shifted);
+    n = n < -1022 ? -1022 : (n > 1023 ? 1023 : n);         // far outside any gain's clamp
+    const double e = exp2(f);
+    return c * fma(e, lost * 0.69314718055994531, e) * __hiloint2double((n + 1023) << 20, 0);
+}
+__device__ __forceinline__ double pow_t(double a, double b) {
+    const Log2Parts l(a);
+    const double bh = coarse(b);
+    return scaled_exp2(1.0, bh * l.k, fma(b, l.m, (b - bh) * l.k));
+}
+#endif
+
 // c a^x b^y for a, b > 0.  In FP64 on the device one exponential serves both
 // powers (Tsit5 FP64, 50,021 Lorenz runs: 996 -> 942 us); in FP32 the two
 // approximate powers side by side have the shorter chain.
@@ -142,10 +173,13 @@ __device__ __forceinline__ float scaled_powers(float c, float a, float x, float 
     return c * pow_t(a, x) * pow_t(b, y);
 }
 __device__ __forceinline__ double scaled_powers(double c, double a, double x, double b, double y) {
-#ifdef CBX_HOST_EMULATION
-    return c * pow_t(a, x) * pow_t(b, y);
+#ifndef CBX_HOST_EMULATION
+    const Log2Parts la(a), lb(b);
+    const double xh = coarse(x), yh = coarse(y);
+    return scaled_exp2(c, xh * la.k + yh * lb.k,
+                       fma(x, la.m, fma(y, lb.m, fma(x - xh, la.k, (y - yh) * lb.k))));
 #else
-    return c * exp2(x * log2(a) + y * log2(b));
+    return c * pow_t(a, x) * pow_t(b, y);
 #endif
 }
 
