@@ -153,6 +153,8 @@ class _Slot:
         self.out_h = {k: torch.zeros(tuple(v.shape), dtype=v.dtype).pin_memory()
                       for k, v in self.bufs.items() if v is not None and k != "work"}
         self.coeff_t = coeff_t
+        # the buffers above (and the driver table) are filled on the current stream
+        self.stream.wait_stream(torch.cuda.current_stream(dev))
         self.pending: Optional[Tuple[int, int]] = None
 
 

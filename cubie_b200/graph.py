@@ -79,6 +79,7 @@ class GraphSolve:
         # per run, whatever the staging buffers hold.
         warm = _native.SolveArgs.from_buffer_copy(self.args)
         warm.max_steps = 1
+        stream.wait_stream(torch.cuda.current_stream(dev))     # the buffers are cleared there
         with torch.cuda.stream(stream):
             self._body(stream, warm)
         stream.synchronize()

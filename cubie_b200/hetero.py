@@ -242,14 +242,19 @@ class HeteroLaunch:
     def launch(self, stream, hargs=None) -> None:
         """Zero the run counters and iteration totals, then launch, on
         ``stream`` (capturable: no allocation, no synchronisation)."""
-        self.work.zero_()
-        for bf in self.bufs:
-            bf["totals"].zero_()
+        torch = _torch()
+        with torch.cuda.stream(stream):
+            self.work.zero_()
+            for bf in self.bufs:
+                bf["totals"].zero_()
         self.module.launch_hetero(hargs or self.hargs, self.owner.block_size, self.grid, stream.cuda_stream)
 
     def timed_launch(self, stream=None) -> float:
         torch = _torch()
-        s0 = stream if stream is not None else torch.cuda.current_stream(torch.device("cuda", self.owner.device))
+        current = torch.cuda.current_stream(torch.device("cuda", self.owner.device))
+        s0 = stream if stream is not None else current
+        if s0 != current:
+            s0.wait_stream(current)     # the inputs, buffers and claim orders are queued there
         e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
         e0.record(s0)
         self.launch(s0)
@@ -266,6 +271,7 @@ class HeteroLaunch:
         warm = _native.HeteroArgs.from_buffer_copy(self.hargs)
         for k in range(self.hargs.n_families):
             warm.family[k].max_steps = 1
+        stream.wait_stream(torch.cuda.current_stream(dev))
         with torch.cuda.stream(stream):
             self.launch(stream, warm)
         stream.synchronize()

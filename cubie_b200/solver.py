@@ -715,7 +715,10 @@ class Solver:
         args = self.make_args(prep, bufs, inits_t, params_t, coeff_t, n_runs, duration, settling_time, t0,
                               dur_t, tol_t, order_t=order_t, zero_work=False)   # fresh buffers
         kernel = self.launch_kind
-        s = stream if stream is not None else torch.cuda.current_stream(dev)
+        current = torch.cuda.current_stream(dev)
+        s = stream if stream is not None else current
+        if s != current:
+            s.wait_stream(current)      # the inputs, cleared buffers and claim order are queued there
         e0 = torch.cuda.Event(enable_timing=True)
         e1 = torch.cuda.Event(enable_timing=True)
         e0.record(s)
