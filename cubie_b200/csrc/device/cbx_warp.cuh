@@ -750,6 +750,9 @@ __device__ __forceinline__ void warp_begin(WarpLane<Cfg>& L, WarpCtx<Cfg>& w, co
         L.y[k] = w.valid(k) ? inits[w.comp(k) * a.run_stride + run] : R(0);
         L.comp[k] = R(0);
     }
+    // the previous run's last right-hand side may still be reading its
+    // parameters on another lane (the register form has no exchange after it)
+    __syncwarp();
 #pragma unroll
     for (int q = 0; q < NP; ++q)
         if (w.lane == q) w.m->p[q] = params[q * a.run_stride + run];
