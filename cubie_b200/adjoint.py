@@ -17,9 +17,9 @@ tableaus for autonomous systems without drivers) gets two extra kernels (``csrc/
 :class:`AdjointIntegrator` drives the two launches;
 :func:`solve_ivp_adjoint` wraps them in a ``torch.autograd.Function`` so a
 torch loss on the returned state tensor back-propagates into the initial
-values and parameters.  Where a record (start state and size) of every
-accepted step of every run fits ``record_share`` of the device's memory,
-the forward launch stores those instead of checkpoints and the backward
+values and parameters.  While every run has a lane of its own and a
+record (start state and size) of every accepted step of every run fits
+``record_share`` of the device's memory, the forward launch stores those instead of checkpoints and the backward
 launch reads them without replaying anything.  Memory:
 ``n_runs * max_ckpts * ckpt_every`` records, or ``n_runs * max_ckpts``
 checkpoint images, one replay segment of ``ckpt_every`` records per run and,
@@ -56,12 +56,16 @@ class AdjointIntegrator:
 
     def _records(self, n_runs: int, record: int, dev):
         """Buffer for a record of every step (``max_ckpts * ckpt_every`` per
-        run), or None where checkpoints and replay are used instead: records
-        above ``record_share`` of the device's memory or of what is free."""
+        run), or None where checkpoints and replay are used instead: more
+        runs than the device has lanes for at once (1,024 an SM at these
+        kernels' registers; cbx_adjoint.cuh has the times), or records above
+        ``record_share`` of the device's memory or of what is free."""
         torch = _torch()
+        device = torch.cuda.get_device_properties(dev)
         cap = self.max_ckpts * self.ckpt_every
         nbytes = n_runs * cap * record
-        if cap >= 2 ** 31 or nbytes > self.record_share * torch.cuda.get_device_properties(dev).total_memory:
+        if (n_runs > 1024 * device.multi_processor_count or cap >= 2 ** 31
+                or nbytes > self.record_share * device.total_memory):
             return None
         try:
             return torch.empty((max(nbytes, 16) // 4,), device=dev, dtype=torch.int32)
@@ -93,38 +97,10 @@ class AdjointIntegrator:
         else:
             adj.tape, adj.tape_flags, adj.step_count = (t.data_ptr() for t in tape)
 
-    def _launch_records(self, prep, args, adj, saved, phase: int, stream) -> None:
-        """Launch the record form in equal parts of at most a lane per run
-        (1,024 an SM at these kernels' registers; cbx_adjoint.cuh has the
-        times), one after the other: each part's arguments start at its first
-        run in every array."""
-        s = self.solver
-        n, size = args.n_runs, np.dtype(s.precision).itemsize
-        cap = self.max_ckpts * self.ckpt_every
-        work = saved["work"]
-        parts = int(work.numel())
-        work.zero_()
-        per = max(1, -(-n // parts))
-        widths = dict(inits=size, params=size, state_out=size, obs_out=size, state_sum_out=size, obs_sum_out=size,
-                      counters_out=4, status_out=4, tol_scale=8)
-        for k, c0 in enumerate(range(0, n, per)):
-            a = _native.SolveArgs.from_buffer_copy(args)
-            g = _native.AdjointArgs.from_buffer_copy(adj)
-            for name, width in widths.items():
-                at = getattr(a, name)
-                if at:
-                    setattr(a, name, at + c0 * width)
-            a.n_runs = min(per, n - c0)
-            a.work_counter = work.data_ptr() + 8 * k
-            g.lane_words = a.n_runs
-            g.seg = saved["records"].data_ptr() + c0 * cap * saved["record"]
-            g.step_count = saved["steps"].data_ptr() + 4 * c0
-            g.ckpt_count += 4 * c0
-            for name in ("grad_state", "grad_inits", "grad_params"):
-                at = getattr(g, name)
-                if at:
-                    setattr(g, name, at + c0 * size)
-            prep["module"].adjoint_launch(a, g, phase, s.block_size, 0, stream, True)
+    @staticmethod
+    def _set_records(adj, records, steps, n_runs: int) -> None:
+        if records is not None:
+            adj.seg, adj.step_count, adj.lane_words = records.data_ptr(), steps.data_ptr(), n_runs
 
     def forward(self, inits_t, params_t, duration: float, settling_time: float = 0.0, t0: float = 0.0,
                 stream=None, tol_scale=None):
@@ -155,11 +131,9 @@ class AdjointIntegrator:
         with torch.cuda.stream(st):
             records = self._records(n_runs, record, dev)
             count = torch.zeros((n_runs,), device=dev, dtype=torch.int32)
-            ckpt = tape = steps = work = None
+            ckpt = tape = steps = None
             if records is not None:
                 steps = torch.empty((n_runs,), device=dev, dtype=torch.int32)
-                lanes = 1024 * torch.cuda.get_device_properties(dev).multi_processor_count
-                work = torch.empty((max(1, -(-n_runs // lanes)),), device=dev, dtype=torch.int64)
             else:
                 ckpt = torch.empty((n_runs * self.max_ckpts * words,), device=dev, dtype=torch.int32)
                 tape = self._tape_buffers(n_runs, tape_entry, dev) if tape_entry > 0 else None
@@ -170,15 +144,12 @@ class AdjointIntegrator:
         adj.ckpt_every = self.ckpt_every
         adj.max_ckpts = self.max_ckpts
         self._set_tape(adj, tape)
+        self._set_records(adj, records, steps, n_runs)
+        prep["module"].adjoint_launch(args, adj, 0, s.block_size, 0, st.cuda_stream, records is not None)
         saved = dict(prep=prep, bufs=bufs, inits=inits_t, params=params_t, tol=tol_t, ckpt=ckpt, count=count,
                      words=words,
-                     record=record, tape=tape, records=records, steps=steps, work=work,
+                     record=record, tape=tape, records=records, steps=steps,
                      n_runs=n_runs, duration=duration, settling_time=settling_time, t0=t0, dev=dev, tdtype=tdtype)
-        if records is None:
-            prep["module"].adjoint_launch(args, adj, 0, s.block_size, 0, st.cuda_stream)
-        else:
-            with torch.cuda.stream(st):
-                self._launch_records(prep, args, adj, saved, 0, st.cuda_stream)
         return bufs["state"], bufs["status"], saved
 
     def backward(self, saved, grad_state, stream=None) -> Tuple["object", "object"]:
@@ -216,11 +187,8 @@ class AdjointIntegrator:
         adj.ckpt_every = self.ckpt_every
         adj.max_ckpts = self.max_ckpts
         self._set_tape(adj, saved["tape"])
-        if saved["records"] is None:
-            prep["module"].adjoint_launch(args, adj, 1, s.block_size, 0, st.cuda_stream)
-        else:
-            with torch.cuda.stream(st):
-                self._launch_records(prep, args, adj, saved, 1, st.cuda_stream)
+        self._set_records(adj, saved["records"], saved["steps"], n_runs)
+        prep["module"].adjoint_launch(args, adj, 1, s.block_size, 0, st.cuda_stream, saved["records"] is not None)
         return gi, (gp if npar > 0 else gp[:0])
 
 

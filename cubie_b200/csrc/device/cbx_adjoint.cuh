@@ -784,16 +784,16 @@ __device__ __forceinline__ void run_adjoint_backward(const cbx_solve_args a, con
 // replayed and no checkpoint or tape exists.  The records are those the
 // replay would produce (the forward's own step starts and sizes).
 //
-// The host launches it over parts in which every run has a lane of its own.
-// The lanes of a warp then walk their steps side by side, and with the runs of
-// one step together ([step][run]) a warp's records are whole lines.  (A run's
-// records together cost a sector per lane and store, 84 us more on the first
-// forward below; more runs than lanes in one launch put the lanes at different
-// steps, and its stores cost more than the replay.)  Checkpoints against
-// records, forward + backward: FitzHugh-Nagumo, 131,072 runs x 130 steps,
-// 1.26 -> 1.04 ms, 300,001 runs in two parts 2.38 -> 2.03, 262,144 runs x 440
-// steps 6.50 -> 6.03; Van der Pol under ROS3P, 8,191 runs 1.08 -> 0.84, 200,000
-// runs 3.95 -> 3.76.  Checkpoints take over where the records do not fit.
+// The host uses it while every run has a lane of its own.  The lanes of a
+// warp then walk their steps side by side, and with the runs of one step
+// together ([step][run]) a warp's records are whole lines.  (A run's records
+// together cost a sector per lane and store, 84 us more on the forward
+// below.)  With more runs than lanes the lanes are at different steps, every
+// layout scatters, and the forward's stores cost more than the replay.
+// Checkpoints against records, forward + backward: FitzHugh-Nagumo, 131,072
+// runs x 130 steps, 1.29 -> 0.98 ms (5,000 runs 0.56 -> 0.48); Van der Pol
+// under ROS3P, 8,191 runs, 1.09 -> 0.89; 300,001 FitzHugh-Nagumo runs 2.35
+// against 2.57, 200,000 Van der Pol runs 3.95 against 4.25 (checkpoints kept).
 template <class Cfg>
 struct RecordWriter {
     using R = typename Cfg::R;

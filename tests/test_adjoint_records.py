@@ -88,7 +88,7 @@ def test_emulated_records_equal_replay(name):
 @pytest.mark.gpu
 @pytest.mark.parametrize("name,precision,mixed,n", [("fhn", np.float32, True, 1001), ("fhn", np.float64, False, 33),
                                                     ("vdp", np.float32, True, 1), ("vdp", np.float32, True, 777),
-                                                    ("fhn", np.float32, True, 151553)])   # two parts
+                                                    ("fhn", np.float32, True, 151553)])   # more runs than lanes
 @pytest.mark.parametrize("every,ckpts", [(64, 64), (7, 90), (3, 4)])
 def test_records_equal_checkpoints(cuda_device, name, precision, mixed, n, every, ckpts):
     import torch
@@ -99,7 +99,7 @@ def test_records_equal_checkpoints(cuda_device, name, precision, mixed, n, every
     for share in (0.125, 0.0):
         integ = AdjointIntegrator(s, ckpt_every=every, max_ckpts=ckpts, record_share=share)
         state, status, saved = integ.forward(x0, p, 8.0)
-        assert (saved["records"] is not None) == (share > 0)
+        assert (saved["records"] is not None) == (share > 0 and n < 151553)
         out.append((state.clone(), status.clone(), *integ.backward(saved, 0.1 * state)))
     (sa, ta, ga, pa), (sb, tb, gb, pb) = out
     assert torch.equal(ta, tb)
