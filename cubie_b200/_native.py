@@ -97,7 +97,7 @@ EXPORTED = (
     "cbx_module_load", "cbx_module_create", "cbx_module_destroy", "cbx_kernel_info",
     "cbx_occupancy", "cbx_solve", "cbx_device_info", "cbx_fp32_peak_probe", "cbx_flush_l2",
     "cbx_solve_noalloc", "cbx_adjoint_info", "cbx_adjoint_tape_bytes", "cbx_adjoint_launch", "cbx_solve_hetero",
-    "cbx_claim_order", "cbx_adjoint_launch_records",
+    "cbx_claim_order", "cbx_adjoint_launch_records", "cbx_adjoint_lanes",
 )
 
 _lib = None
@@ -162,6 +162,7 @@ def lib():
         L.cbx_adjoint_launch.argtypes = [ctypes.c_void_p, ctypes.POINTER(SolveArgs), ctypes.POINTER(AdjointArgs),
                                          ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_void_p]
         L.cbx_adjoint_launch_records.argtypes = L.cbx_adjoint_launch.argtypes
+        L.cbx_adjoint_lanes.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.POINTER(ctypes.c_longlong)]
         _lib = L
         return L
 
@@ -272,6 +273,12 @@ class Module:
         """Bytes of one step-size tape entry (0: the module keeps no tape)."""
         v = ctypes.c_longlong()
         _check(lib().cbx_adjoint_tape_bytes(self._handle, ctypes.byref(v)), "cbx_adjoint_tape_bytes")
+        return v.value
+
+    def adjoint_lanes(self, block: int) -> int:
+        """Runs that both kernels of the record form hold at once."""
+        v = ctypes.c_longlong()
+        _check(lib().cbx_adjoint_lanes(self._handle, block, ctypes.byref(v)), "cbx_adjoint_lanes")
         return v.value
 
     def adjoint_launch(self, args: SolveArgs, adj: AdjointArgs, phase: int, block: int, grid: int = 0,

@@ -54,18 +54,21 @@ class AdjointIntegrator:
         self.max_ckpts = int(max_ckpts)
         self.record_share = float(record_share)
 
-    def _records(self, n_runs: int, record: int, dev):
+    def _records(self, prep, n_runs: int, record: int, dev):
         """Buffer for a record of every step (``max_ckpts * ckpt_every`` per
         run), or None where checkpoints and replay are used instead: more
-        runs than the device has lanes for at once (1,024 an SM at these
-        kernels' registers; cbx_adjoint.cuh has the times), or records above
-        ``record_share`` of the device's memory or of what is free."""
+        runs than the record kernels hold at once (cbx_adjoint.cuh has the
+        times), or records above ``record_share`` of the device's memory or of
+        what is free."""
         torch = _torch()
-        device = torch.cuda.get_device_properties(dev)
         cap = self.max_ckpts * self.ckpt_every
         nbytes = n_runs * cap * record
-        if (n_runs > 1024 * device.multi_processor_count or cap >= 2 ** 31
-                or nbytes > self.record_share * device.total_memory):
+        if cap >= 2 ** 31 or nbytes > self.record_share * torch.cuda.get_device_properties(dev).total_memory:
+            return None
+        lanes = prep.get("record_lanes")
+        if lanes is None:
+            lanes = prep["record_lanes"] = prep["module"].adjoint_lanes(self.solver.block_size)
+        if n_runs > lanes:
             return None
         try:
             return torch.empty((max(nbytes, 16) // 4,), device=dev, dtype=torch.int32)
@@ -129,7 +132,7 @@ class AdjointIntegrator:
         lane, record, tape_entry = self.sizes(prep)
         words = lane // 4
         with torch.cuda.stream(st):
-            records = self._records(n_runs, record, dev)
+            records = self._records(prep, n_runs, record, dev)
             count = torch.zeros((n_runs,), device=dev, dtype=torch.int32)
             ckpt = tape = steps = None
             if records is not None:

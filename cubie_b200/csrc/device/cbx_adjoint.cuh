@@ -784,16 +784,23 @@ __device__ __forceinline__ void run_adjoint_backward(const cbx_solve_args a, con
 // replayed and no checkpoint or tape exists.  The records are those the
 // replay would produce (the forward's own step starts and sizes).
 //
-// The host uses it while every run has a lane of its own.  The lanes of a
-// warp then walk their steps side by side, and with the runs of one step
-// together ([step][run]) a warp's records are whole lines.  (A run's records
-// together cost a sector per lane and store, 84 us more on the forward
-// below.)  With more runs than lanes the lanes are at different steps, every
-// layout scatters, and the forward's stores cost more than the replay.
-// Checkpoints against records, forward + backward: FitzHugh-Nagumo, 131,072
-// runs x 130 steps, 1.29 -> 0.98 ms (5,000 runs 0.56 -> 0.48); Van der Pol
-// under ROS3P, 8,191 runs, 1.09 -> 0.89; 300,001 FitzHugh-Nagumo runs 2.35
-// against 2.57, 200,000 Van der Pol runs 3.95 against 4.25 (checkpoints kept).
+// The host uses it while every run has a lane of its own, by the occupancy of
+// these two kernels (cbx_adjoint_lanes).  The lanes of a warp then start
+// together, and with the runs of one step together ([step][run]) the records
+// of a warp whose lanes keep step are whole lines.  (A run's records together
+// cost a sector per lane and store, 84 us more on the first forward below.)
+// More runs than lanes put the lanes at different steps, every layout scatters,
+// and the forward's stores cost more than the replay.  Checkpoints against
+// records, forward + backward:
+//   FitzHugh-Nagumo, all spiking: 131,072 runs x 169 steps 1.05 -> 0.81 ms;
+//     300,001 runs 2.35 against 2.57 (checkpoints kept);
+//   some spiking, some not, 429 +- 106 steps: 2,000 runs 1.10 -> 0.86, 8,191
+//     1.15 -> 0.99, 40,000 1.44 -> 1.41; from there the drifting lanes' stores
+//     show: 80,000 2.12 -> 2.17, 131,072 3.04 -> 3.24; FP64, 75,776 runs
+//     4.02 -> 2.83;
+//   Van der Pol under ROS3P, 8,191 runs x 257 steps 0.61 -> 0.51, 131,072
+//     1.54 -> 1.12; 836 +- 84 steps, 30,000 runs 1.74 -> 1.52, 131,072
+//     4.26 -> 3.98; 200,000 runs 3.95 against 4.25 (checkpoints kept).
 template <class Cfg>
 struct RecordWriter {
     using R = typename Cfg::R;

@@ -603,6 +603,27 @@ extern "C" int cbx_adjoint_launch(cbx_module* module, const cbx_solve_args* args
     return adjoint_launch(module, args, adj, false, phase, block, grid, stream);
 }
 
+extern "C" int cbx_adjoint_lanes(cbx_module* module, int block, long long* lanes) {
+    if (!module || !lanes || block <= 0 || block > 1024 || (block % 32) != 0)
+        return fail(CBX_ERR_ARGUMENT, "bad module, block size (%d) or output", block);
+    if (!load_driver()) return fail(CBX_ERR_NO_DEVICE, "CUDA driver library is not available");
+    CUcontext cur = nullptr;
+    g_drv.cuCtxGetCurrent(&cur);
+    int rc = cur == module->context ? CBX_OK : check_cu(g_drv.cuCtxSetCurrent(module->context), "cuCtxSetCurrent");
+    if (!rc) rc = resolve_adjoint(module);
+    if (rc) return rc;
+    *lanes = 0;
+    for (int k = 2; k < 4; ++k) {
+        int per_sm = 0;
+        rc = check_cu(g_drv.cuOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, module->adj[k], block, 0),
+                      "cuOccupancyMaxActiveBlocksPerMultiprocessor");
+        if (rc) return rc;
+        const long long n = (long long)per_sm * module->sm_count * block;
+        if (k == 2 || n < *lanes) *lanes = n;
+    }
+    return CBX_OK;
+}
+
 extern "C" int cbx_adjoint_launch_records(cbx_module* module, const cbx_solve_args* args,
                                           const cbx_adjoint_args* adj, int phase, int block, int grid, void* stream) {
     return adjoint_launch(module, args, adj, true, phase, block, grid, stream);

@@ -114,6 +114,30 @@ def test_records_equal_checkpoints(cuda_device, name, precision, mixed, n, every
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("name,precision,mixed", [("fhn", np.float32, True), ("fhn", np.float64, False),
+                                                  ("vdp", np.float32, True)])
+def test_records_while_every_run_has_a_lane(cuda_device, name, precision, mixed):
+    """The record form ends at the runs its kernels hold at once, which their
+    registers decide (FP64 takes twice as many)."""
+    import torch
+    from cubie_b200.adjoint import AdjointIntegrator
+    s = _solver(name, precision, mixed)
+    integ = AdjointIntegrator(s, ckpt_every=3, max_ckpts=4)
+    x0, p = (torch.tensor(v.astype(precision), device="cuda") for v in _batch(name, 2, 3))
+    _, _, saved = integ.forward(x0, p, 0.5)
+    lanes = saved["prep"]["record_lanes"]
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert lanes % (sms * s.block_size) == 0 and 256 <= lanes // sms <= 2048
+    assert lanes // sms <= (640 if precision == np.float64 else 1280)      # 96 and 48 registers
+    for n in (lanes, lanes + 1):
+        x, q = x0[:, :1].repeat(1, n), p[:, :1].repeat(1, n)
+        state, status, saved = integ.forward(x, q, 0.5)
+        assert (saved["records"] is not None) == (n == lanes)
+        gi, gp = integ.backward(saved, torch.ones_like(state))
+        assert torch.equal(gi, gi[:, :1].expand_as(gi)) and torch.equal(gp, gp[:, :1].expand_as(gp))
+
+
+@pytest.mark.gpu
 def test_autograd_passes_release_their_records(cuda_device):
     import gc
     import torch
