@@ -31,12 +31,29 @@ status 32 (step budget), like ``max_steps``.
 
 from __future__ import annotations
 
-from typing import Optional, Tuple
+from typing import Dict, Optional, Tuple
 
 import numpy as np
 
 from . import _native
 from .solver import Solver, _torch
+
+
+# Records take about twice the memory of checkpoints, tape and segment, and a
+# training loop may hold two forward passes at once, so a buffer above
+# RECORDS_UNASKED bytes has to fit RECORDS_OF_FREE times into what is free.
+RECORDS_UNASKED = 1 << 30
+RECORDS_OF_FREE = 4
+
+
+def _free_bytes(dev, enough: int) -> int:
+    """Free device memory, with what torch's allocator holds unused counted
+    in where the device alone has less than ``enough``."""
+    torch = _torch()
+    free = torch.cuda.mem_get_info(dev)[0]
+    if free < enough:
+        free += torch.cuda.memory_reserved(dev) - torch.cuda.memory_allocated(dev)
+    return free
 
 
 class AdjointIntegrator:
@@ -53,13 +70,15 @@ class AdjointIntegrator:
         self.ckpt_every = int(ckpt_every)
         self.max_ckpts = int(max_ckpts)
         self.record_share = float(record_share)
+        self._roomy: Dict[int, bool] = {}       # record buffer sizes asked for: whether memory had room
 
     def _records(self, prep, n_runs: int, record: int, dev):
         """Buffer for a record of every step (``max_ckpts * ckpt_every`` per
         run), or None where checkpoints and replay are used instead: more
         runs than the record kernels hold at once (cbx_adjoint.cuh has the
-        times), or records above ``record_share`` of the device's memory or of
-        what is free."""
+        times), records above ``record_share`` of the device's memory, or large
+        ones above a quarter of what was free when this integrator first met
+        their size (asked once: 80 us)."""
         torch = _torch()
         cap = self.max_ckpts * self.ckpt_every
         nbytes = n_runs * cap * record
@@ -70,6 +89,12 @@ class AdjointIntegrator:
             lanes = prep["record_lanes"] = prep["module"].adjoint_lanes(self.solver.block_size)
         if n_runs > lanes:
             return None
+        if nbytes > RECORDS_UNASKED:
+            if nbytes not in self._roomy:
+                enough = RECORDS_OF_FREE * nbytes
+                self._roomy[nbytes] = _free_bytes(dev, enough) >= enough
+            if not self._roomy[nbytes]:
+                return None
         try:
             return torch.empty((max(nbytes, 16) // 4,), device=dev, dtype=torch.int32)
         except torch.cuda.OutOfMemoryError:
