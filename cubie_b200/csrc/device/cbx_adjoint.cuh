@@ -792,23 +792,58 @@ __device__ __forceinline__ void run_adjoint_backward(const cbx_solve_args a, con
 // More runs than lanes put the lanes at different steps, every layout scatters,
 // and the forward's stores cost more than the replay.  Checkpoints against
 // records, forward + backward:
-//   FitzHugh-Nagumo, all spiking: 131,072 runs x 169 steps 1.05 -> 0.81 ms;
+//   FitzHugh-Nagumo, all spiking: 131,072 runs x 169 steps 1.02 -> 0.80 ms;
 //     300,001 runs 2.35 against 2.57 (checkpoints kept);
 //   some spiking, some not, 429 +- 106 steps: 2,000 runs 1.10 -> 0.86, 8,191
-//     1.15 -> 0.99, 40,000 1.44 -> 1.41; from there the drifting lanes' stores
-//     show: 80,000 2.12 -> 2.17, 131,072 3.04 -> 3.24; FP64, 75,776 runs
-//     4.02 -> 2.83;
-//   Van der Pol under ROS3P, 8,191 runs x 257 steps 0.61 -> 0.51, 131,072
-//     1.54 -> 1.12; 836 +- 84 steps, 30,000 runs 1.74 -> 1.52, 131,072
-//     4.26 -> 3.98; 200,000 runs 3.95 against 4.25 (checkpoints kept).
+//     1.13 -> 0.97, 40,000 1.45 -> 1.39, 80,000 2.10 -> 2.00; FP64, 75,776
+//     runs 4.02 -> 2.83;
+//   Van der Pol under ROS3P, 8,191 runs x 257 steps 0.60 -> 0.46; 836 +- 84
+//     steps, 30,000 runs 1.71 -> 1.48; 200,000 runs 3.95 against 4.25
+//     (checkpoints kept).
+//
+// Where the records lie: the runs of one step together, [step][run]; with
+// 16-byte records, more than 65,536 runs and an even limit of steps the runs of
+// a pair of steps together, [step / 2][run][step % 2].  A record of a drifting
+// lane is half a 32-byte sector.  One step of that many runs is a megabyte, so
+// the steps the lanes are at spread over more than the L2 holds, and [step][run]
+// moves half-empty sectors to and from memory; a pair fills its sector within
+// two steps of its run.  [step][run] against pairs (checkpoints), 131,072 runs:
+// FitzHugh-Nagumo, 429 +- 106 steps 3.24 -> 2.94 ms (3.05), Van der Pol,
+// 836 +- 84 steps 3.95 -> 3.31 (4.24), 257 +- 30 steps 1.08 -> 1.03 (1.53); runs
+// that all keep step, whose stores were whole lines, 0.73 -> 0.80 (1.02).  At
+// 40,000 runs pairs gain nothing (1.37, 1.39), and groups of four or eight steps
+// cost the runs that keep step more than they save the others (0.84 and 0.92
+// against 2.90 and 2.96).  Each kernel holds its loop once for either layout.
+template <class Cfg, bool PAIRS>
+struct RecordPlace {
+    using R = typename Cfg::R;
+    static constexpr int F = SegRecord<Cfg>::F;
+    // record j of a run, and the values between records j and j + 1
+    static __device__ __forceinline__ R* at(const cbx_adjoint_args& g, long long run, int j) {
+        R* records = static_cast<R*>(g.seg);
+        if constexpr (PAIRS) return records + ((j & ~1) * g.lane_words + 2 * run + (j & 1)) * F;
+        else return records + (j * g.lane_words + run) * F;
+    }
+    static __device__ __forceinline__ long long step(const cbx_adjoint_args& g, int j) {
+        if constexpr (PAIRS) return (j & 1) ? (2 * g.lane_words - 1) * F : F;
+        else return g.lane_words * F;
+    }
+};
+
 template <class Cfg>
+__device__ __forceinline__ bool records_in_pairs(const cbx_adjoint_args& g) {
+    return SegRecord<Cfg>::F * int(sizeof(typename Cfg::R)) < 32 && g.lane_words > 65536 &&
+           ((g.max_ckpts * g.ckpt_every) & 1) == 0;
+}
+
+template <class Cfg, bool PAIRS>
 struct RecordWriter {
     using R = typename Cfg::R;
     using C = typename Cfg::C;
     using Rec = SegRecord<Cfg>;
     static constexpr bool ACTIVE = true;
+    const cbx_adjoint_args& g;
     R* next;
-    long long step_step;
     int count;
     __device__ __forceinline__ void accepted(const Lane<Cfg>& L, C dt_eff, int row) {
         R rec[Rec::F];
@@ -820,28 +855,27 @@ struct RecordWriter {
 #pragma unroll
         for (int k = Rec::H_AT + 1; k < Rec::F; ++k) rec[k] = R(0);
         Rec::store(next, rec);
-        next += step_step;
+        next += RecordPlace<Cfg, PAIRS>::step(g, count);
         ++count;
     }
 };
 
-template <class Cfg>
-__device__ __forceinline__ void run_adjoint_forward_records(const cbx_solve_args a, const cbx_adjoint_args g) {
+template <class Cfg, bool PAIRS>
+__device__ __forceinline__ void forward_records(const cbx_solve_args& a, const cbx_adjoint_args& g) {
     using R = typename Cfg::R;
     __shared__ BlockTotals bt;
     totals_begin(&bt);
     Lane<Cfg> L;
     bool active = false, exhausted = !lane_in_use(a.n_runs);
     const int cap = g.max_ckpts * g.ckpt_every;
-    const long long step_step = g.lane_words * SegRecord<Cfg>::F;   // values from a run's record to its next
-    RecordWriter<Cfg> rec{nullptr, step_step, 0};
+    RecordWriter<Cfg, PAIRS> rec{g, nullptr, 0};
     while (true) {
         if (!active && !exhausted) {
             const long long run = claim_run(a.work_counter);
             if (run < a.n_runs) {
                 lane_begin<Cfg>(L, a, run);
                 active = true;
-                rec.next = static_cast<R*>(g.seg) + run * SegRecord<Cfg>::F;
+                rec.next = RecordPlace<Cfg, PAIRS>::at(g, run, 0);
                 rec.count = 0;
             } else {
                 exhausted = true;
@@ -855,7 +889,7 @@ __device__ __forceinline__ void run_adjoint_forward_records(const cbx_solve_args
                     L.status |= MAX_LOOP_ITERS_EXCEEDED;
                     done = true;
                 } else {
-                    done = lane_iterate<Cfg, RecordWriter<Cfg>>(L, a, &rec);
+                    done = lane_iterate<Cfg, RecordWriter<Cfg, PAIRS>>(L, a, &rec);
                 }
             }
         } while (!__any_sync(0xffffffffu, done));
@@ -871,15 +905,14 @@ __device__ __forceinline__ void run_adjoint_forward_records(const cbx_solve_args
 
 // Reverse sweep over the records: every lane walks its own run backwards, the
 // next (earlier) record and the next saved row's loss gradient in flight.
-template <class Cfg>
-__device__ __forceinline__ void run_adjoint_backward_records(const cbx_solve_args a, const cbx_adjoint_args g) {
+template <class Cfg, bool PAIRS>
+__device__ __forceinline__ void backward_records(const cbx_solve_args& a, const cbx_adjoint_args& g) {
     using R = typename Cfg::R;
     using C = typename Cfg::C;
     using Adj = StepAdjoint<Cfg, Cfg::ALGO>;
     using Rec = SegRecord<Cfg>;
     constexpr int N = Cfg::N, NP = Cfg::NP, F = Rec::F, NPP = NP > 0 ? NP : 1;
     const long long s = a.run_stride;
-    const long long step_step = g.lane_words * F;
     const R* params = static_cast<const R*>(a.params);
     R lam[N], p[NPP], nxt[F];
     C pbar[NPP];
@@ -905,7 +938,7 @@ __device__ __forceinline__ void run_adjoint_backward_records(const cbx_solve_arg
                 j = g.step_count[run] - 1;
                 rows_end = g.ckpt_count[run];
                 if (j >= 0) {
-                    rec_at = static_cast<const R*>(g.seg) + run * F + j * step_step;
+                    rec_at = RecordPlace<Cfg, PAIRS>::at(g, run, j);
                     Rec::load(rec_at, nxt);
                     row_next.load(a, g, rows_end - 1, run);
                 }
@@ -919,7 +952,7 @@ __device__ __forceinline__ void run_adjoint_backward_records(const cbx_solve_arg
 #pragma unroll
             for (int k = 0; k < F; ++k) rec_j[k] = nxt[k];
             if (j > 0) {
-                rec_at -= step_step;
+                rec_at -= RecordPlace<Cfg, PAIRS>::step(g, j - 1);
                 Rec::load(rec_at, nxt);
             }
             const R hs = rec_j[Rec::H_AT];
@@ -948,6 +981,17 @@ __device__ __forceinline__ void run_adjoint_backward_records(const cbx_solve_arg
             active = false;
         }
     }
+}
+
+template <class Cfg>
+__device__ __forceinline__ void run_adjoint_forward_records(const cbx_solve_args& a, const cbx_adjoint_args& g) {
+    if (records_in_pairs<Cfg>(g)) forward_records<Cfg, true>(a, g);
+    else forward_records<Cfg, false>(a, g);
+}
+template <class Cfg>
+__device__ __forceinline__ void run_adjoint_backward_records(const cbx_solve_args& a, const cbx_adjoint_args& g) {
+    if (records_in_pairs<Cfg>(g)) backward_records<Cfg, true>(a, g);
+    else backward_records<Cfg, false>(a, g);
 }
 
 }  // namespace cbx

@@ -76,8 +76,8 @@ typedef struct cbx_solve_args {
  *
  * The record form (cbx_adjoint_launch_records) uses seg, step_count,
  * ckpt_count and the gradient pointers only: the forward launch stores one
- * record per accepted step, seg [cap][lane_words][record_bytes] with
- * lane_words >= n_runs, and in ckpt_count the rows each run saved; the
+ * record per accepted step, seg [cap][lane_words][record_bytes] in size (the
+ * kernels may group the steps otherwise) with lane_words >= n_runs, and in ckpt_count the rows each run saved; the
  * reverse sweep reads them and replays nothing.
  */
 typedef struct cbx_adjoint_args {

@@ -47,20 +47,21 @@ def _batch(name, n, seed=0):
     return np.stack([rng.uniform(1, 2, n), rng.uniform(-1, 1, n)]), rng.uniform(0.5, 3.0, (1, n))
 
 
-@pytest.mark.parametrize("name", ["fhn", "vdp"])
-def test_emulated_records_equal_replay(name):
+def _emulated_against_replay(name, every, ckpts, lanes=None):
+    """Both forms in emulation: the same bits; returns (steps, statuses)."""
     from emu import compile_emulated, run_emulated_adjoint
     from cubie_b200 import _native
     s = _solver(name)
     x0, p = _batch(name, 5)
-    T, every, ckpts = 6.0, 4, 64
+    T = 6.0
     state, status, gi, gp = run_emulated_adjoint(s, x0, p, T, lambda y: 0.1 * y, every, ckpts)
     prep = s.prepare(T, 0.0, 0.0, None, None, load=False)
     lib = compile_emulated(prep["gen"].source + DRIVER)
     n, cap = x0.shape[1], every * ckpts
+    lanes = lanes or n
     x, q = np.ascontiguousarray(x0, np.float32), np.ascontiguousarray(p, np.float32)
     out = dict(state=np.zeros_like(state), status=np.zeros_like(status), work=np.zeros(2, np.uint64),
-               seg=np.zeros(n * cap * int(lib.emu_record_bytes()) // 8 + 2), count=np.zeros(n, np.int32),
+               seg=np.full(lanes * cap * int(lib.emu_record_bytes()) // 8 + 2, np.nan), count=np.zeros(n, np.int32),
                steps=np.zeros(n, np.int32), gi=np.zeros_like(gi), gp=np.zeros((p.shape[0], n), np.float32))
     grad = np.ascontiguousarray(0.1 * state, np.float32)
     a = _native.SolveArgs()
@@ -72,17 +73,64 @@ def test_emulated_records_equal_replay(name):
     g = _native.AdjointArgs()
     g.seg, g.ckpt_count, g.step_count = (out[k].ctypes.data for k in ("seg", "count", "steps"))
     g.ckpt_every, g.max_ckpts = every, ckpts
-    g.lane_words = n
+    g.lane_words = lanes
     g.grad_state, g.grad_inits, g.grad_params = grad.ctypes.data, out["gi"].ctypes.data, out["gp"].ctypes.data
     lib.emu_records(ctypes.byref(a), ctypes.byref(g), 0, 32)
     out["work"][:] = 0
     lib.emu_records(ctypes.byref(a), ctypes.byref(g), 1, 32)
     # one compiler, no contraction: the same bits
-    assert out["steps"].min() > 2 * every
     np.testing.assert_array_equal(out["state"], state)
     np.testing.assert_array_equal(out["status"], status)
     np.testing.assert_array_equal(out["gi"], gi)
     np.testing.assert_array_equal(out["gp"], gp)
+    assert np.all(np.isnan(out["seg"][-2:]))          # nothing past the records
+    return out["steps"], status
+
+
+@pytest.mark.parametrize("name", ["fhn", "vdp"])
+def test_emulated_records_equal_replay(name):
+    steps, _ = _emulated_against_replay(name, 4, 64)
+    assert steps.min() > 2 * 4
+
+
+# records of more than 65,536 lanes lie in pairs of steps where the limit of
+# steps is even; runs that stop at the limit and runs that end before it
+@pytest.mark.parametrize("name", ["fhn", "vdp"])
+@pytest.mark.parametrize("every,ckpts", [(4, 32), (3, 5), (1, 2), (7, 2)])
+def test_emulated_pairs_equal_replay(name, every, ckpts):
+    steps, status = _emulated_against_replay(name, every, ckpts, lanes=65537)
+    if every * ckpts <= 15:
+        assert np.all(steps == every * ckpts) and np.all(status == 32)
+    else:
+        assert steps.min() > 2 * every
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name,precision,mixed", [("fhn", np.float32, True), ("vdp", np.float32, True),
+                                                  ("fhn", np.float64, False)])
+@pytest.mark.parametrize("n", [65536, 65537])
+@pytest.mark.parametrize("every,ckpts", [(64, 16), (3, 5)])
+def test_record_layouts_equal_checkpoints_run_by_run(cuda_device, name, precision, mixed, n, every, ckpts):
+    """Both record layouts against checkpoints, every run by itself: states,
+    statuses and gradients, with a tolerance scale per run."""
+    import torch
+    from cubie_b200.adjoint import AdjointIntegrator
+    s = _solver(name, precision, mixed)
+    x0, p = (torch.tensor(v.astype(precision), device="cuda") for v in _batch(name, n, 3))
+    scale = torch.tensor(10.0 ** np.random.default_rng(4).uniform(-0.5, 0.5, n), device="cuda")
+    out = []
+    for share in (0.125, 0.0):
+        integ = AdjointIntegrator(s, ckpt_every=every, max_ckpts=ckpts, record_share=share)
+        state, status, saved = integ.forward(x0, p, 8.0, tol_scale=scale)
+        assert (saved["records"] is not None) == (share > 0)
+        out.append((state.clone(), status.clone(), *integ.backward(saved, 0.1 * state)))
+    (sa, ta, ga, pa), (sb, tb, gb, pb) = out
+    assert torch.equal(ta, tb) and bool((ta != 0).any()) == (every == 3)
+    # as in test_records_equal_checkpoints, each run against its own size
+    tol = 100 * 200 * (1.2e-7 if precision == np.float32 else 2.3e-16)
+    for u, v in ((sa, sb), (ga, gb), (pa, pb)):
+        u, v = u.reshape(-1, n).double(), v.reshape(-1, n).double()
+        assert float(((u - v).norm(dim=0) / v.norm(dim=0).clamp(min=1e-3)).max()) <= tol
 
 
 @pytest.mark.gpu
