@@ -160,8 +160,14 @@ class AdjointIntegrator:
             records = self._records(prep, n_runs, record, dev)
             count = torch.zeros((n_runs,), device=dev, dtype=torch.int32)
             ckpt = tape = steps = None
+            params_kept, tol_kept = params_t, tol_t
             if records is not None:
                 steps = torch.empty((n_runs,), device=dev, dtype=torch.int32)
+                # checkpoints hold each run's parameters and tolerance scale,
+                # records do not: the reverse sweep reads copies, whatever the
+                # caller writes to its own tensors meanwhile
+                params_kept = params_t.clone()
+                tol_kept = None if tol_t is None else tol_t.clone()
             else:
                 ckpt = torch.empty((n_runs * self.max_ckpts * words,), device=dev, dtype=torch.int32)
                 tape = self._tape_buffers(n_runs, tape_entry, dev) if tape_entry > 0 else None
@@ -174,9 +180,8 @@ class AdjointIntegrator:
         self._set_tape(adj, tape)
         self._set_records(adj, records, steps, n_runs)
         prep["module"].adjoint_launch(args, adj, 0, s.block_size, 0, st.cuda_stream, records is not None)
-        saved = dict(prep=prep, bufs=bufs, inits=inits_t, params=params_t, tol=tol_t, ckpt=ckpt, count=count,
-                     words=words,
-                     record=record, tape=tape, records=records, steps=steps,
+        saved = dict(prep=prep, bufs=bufs, inits=inits_t, params=params_kept, tol=tol_kept, ckpt=ckpt, count=count,
+                     words=words, record=record, tape=tape, records=records, steps=steps,
                      n_runs=n_runs, duration=duration, settling_time=settling_time, t0=t0, dev=dev, tdtype=tdtype)
         return bufs["state"], bufs["status"], saved
 

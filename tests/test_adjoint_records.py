@@ -186,6 +186,28 @@ def test_records_while_every_run_has_a_lane(cuda_device, name, precision, mixed)
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("name", ["fhn", "vdp"])
+@pytest.mark.parametrize("share", [0.125, 0.0])
+def test_inputs_written_between_forward_and_backward(cuda_device, name, share):
+    """The gradient is the forward pass's, whatever the caller writes to the
+    initial values, parameters and tolerance scales after it."""
+    import torch
+    from cubie_b200.adjoint import AdjointIntegrator
+    s = _solver(name)
+    out = []
+    for write in (False, True):
+        x0, p = (torch.tensor(v.astype(np.float32), device="cuda") for v in _batch(name, 300, 3))
+        scale = torch.ones(300, dtype=torch.float64, device="cuda")
+        integ = AdjointIntegrator(s, record_share=share)
+        state, _, saved = integ.forward(x0, p, 4.0, tol_scale=scale)
+        if write:
+            x0.fill_(7.0), p.mul_(1.5), scale.fill_(1e-3)
+        out.append(integ.backward(saved, 0.1 * state))
+    for a, b in zip(*out):
+        assert torch.equal(a, b)
+
+
+@pytest.mark.gpu
 def test_records_leave_room_for_the_caller(cuda_device, monkeypatch):
     """Large records need four times their size free (the device's, or unused
     in torch's pool); the answer stays with the integrator and the size."""
