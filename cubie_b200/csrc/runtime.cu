@@ -393,7 +393,9 @@ int cbx_solve(cbx_module* module, const cbx_solve_args* args, int kernel, int bl
                 // schedulers are idle.  128-thread blocks, packed against one
                 // block per SM: Lorenz, 96 runs 75 -> 63 us, 4,096 runs
                 // saving rows 224 -> 191; Van der Pol, 5,001 runs with GMRES
-                // 2.87 -> 2.71 ms, 10,001 under Radau IIA 3.02 -> 2.85.  From
+                // 2.87 -> 2.71 ms, 10,001 under Radau IIA 3.02 -> 2.85.  (That
+                // reaches every SM with blocks of at most 128 threads; larger
+                // blocks are as many warps on fewer SMs.)  From
                 // two warps per scheduler on the warps slow each other (the
                 // 4,096 runs: 205 us at two, 237 at three).
                 const long long spread = (long long)module->sm_count * 128 / block;

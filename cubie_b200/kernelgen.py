@@ -436,9 +436,15 @@ def generate_hetero_kernel(families: Sequence[Tuple[SymbolicODE, KernelSpec, Gen
         raise ValueError("one to eight families per heterogeneous launch")
     block = int(families[0][1].block_size)
     lines = ["// generated by cubie_b200.kernelgen (heterogeneous batch); do not edit"]
-    # the register allowance of the family that profits from one (Lorenz
-    # DP54, Van der Pol and Robertson under direct ROS3P, 50,000 runs each:
-    # 2.09 -> 1.90 ms)
+    # the register allowance of the family that profits from one, also where
+    # the others are explicit: their loops alone lose a little by it, the mixed
+    # kernel holds the largest family's registers for all anyway.  Without
+    # against with the bound: Lorenz, Van der Pol and Robertson (direct ROS3P),
+    # 50,000 runs each 2.09 -> 1.90 ms; Lorenz and FitzHugh-Nagumo (explicit),
+    # 100,000 each, with 2,000 Van der Pol runs 0.78 -> 0.74, with 50,000
+    # 0.91 -> 0.86; 200,000 Lorenz with 2,000 Van der Pol 0.77 -> 0.76; 150,000
+    # Lorenz with 5,000 Radau IIA5 runs 24.3 -> 21.3; FP64 Lorenz, 100,000,
+    # with 2,000 Van der Pol 1.70, 1.70 ms
     min_blocks = max(thread_min_blocks(replace(spec, block_size=block, min_blocks_per_sm=0, max_registers=0))
                      for _, spec, _ in families)
     if min_blocks:
@@ -468,7 +474,18 @@ def warp_min_blocks(spec: KernelSpec, warp_code) -> int:
     1.48 / 1.90, 256 1.79 / 1.33 / 1.60, 288 2.56 / 2.14 / 2.77, 320 2.25 /
     2.03 / 2.50, 384 1.37 / 1.96 / 2.60, 512 2.03 / 2.93 / 3.94: 16 warps
     where the lane's vectors then just fit 128 registers, 12 where they fit
-    168, and no bound where it would spill them or is not needed."""
+    168, and no bound where it would spill them or is not needed.
+
+    Those are times of some thousand runs, in which full rounds of the
+    resident warps count; the rate (resident warps per SM over a round's time)
+    draws the same lines.  Warps per SM over the ms of a round, own choice / 12 /
+    16 warps, FP32: cable of 192 states (328 bytes a lane) 26 / 27 / 32, although
+    2,500 runs fill two rounds either way and take 8 % longer by the bound;
+    rings of FitzHugh-Nagumo cells, 192 states (320) 36 / 35 / 37, 256 (424)
+    31 / 30 / 29, 320 (528) 21 / 26 / 24.  FP64: cables of 96 states (416)
+    11.9 / 15.0 / 13.9 and 128 (416) 13.1 / 15.0 / 16.9, ring of 128 (432) 15.3 /
+    19.0 / 18.2; without a bound by this rule, cables of 160 states (568) 6.7 /
+    7.2 / 8.5, 192 (656) 7.4 / 8.3 / 6.8, 256 (832) 7.4 / 6.7 / 8.0."""
     if int(spec.min_blocks_per_sm):
         return int(spec.min_blocks_per_sm) if int(spec.min_blocks_per_sm) > 1 else 0
     if not warp_code.register_slots or spec.max_registers:
