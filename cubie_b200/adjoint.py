@@ -41,19 +41,18 @@ from .solver import Solver, _torch
 
 # Records take about twice the memory of checkpoints, tape and segment, and a
 # training loop may hold two forward passes at once, so a buffer above
-# RECORDS_UNASKED bytes has to fit RECORDS_OF_FREE times into what is free.
+# RECORDS_UNASKED bytes has to fit RECORDS_OF_FREE times into the device memory
+# that torch's tensors leave.
 RECORDS_UNASKED = 1 << 30
 RECORDS_OF_FREE = 4
 
 
-def _free_bytes(dev, enough: int) -> int:
-    """Free device memory, with what torch's allocator holds unused counted
-    in where the device alone has less than ``enough``."""
+def _free_bytes(dev) -> int:
+    """Device memory without what torch's tensors hold: the allocator's own
+    count (the driver's answer takes 80 us, and milliseconds on a busy host)."""
     torch = _torch()
-    free = torch.cuda.mem_get_info(dev)[0]
-    if free < enough:
-        free += torch.cuda.memory_reserved(dev) - torch.cuda.memory_allocated(dev)
-    return free
+    held = torch.cuda.memory_stats_as_nested_dict(dev).get("allocated_bytes", {}).get("all", {}).get("current", 0)
+    return torch.cuda.get_device_properties(dev).total_memory - held
 
 
 class AdjointIntegrator:
@@ -77,8 +76,8 @@ class AdjointIntegrator:
         run), or None where checkpoints and replay are used instead: more
         runs than the record kernels hold at once (cbx_adjoint.cuh has the
         times), records above ``record_share`` of the device's memory, or large
-        ones above a quarter of what was free when this integrator first met
-        their size (asked once: 80 us)."""
+        ones above a quarter of what torch's tensors left when this integrator
+        first met their size."""
         torch = _torch()
         cap = self.max_ckpts * self.ckpt_every
         nbytes = n_runs * cap * record
@@ -91,8 +90,7 @@ class AdjointIntegrator:
             return None
         if nbytes > RECORDS_UNASKED:
             if nbytes not in self._roomy:
-                enough = RECORDS_OF_FREE * nbytes
-                self._roomy[nbytes] = _free_bytes(dev, enough) >= enough
+                self._roomy[nbytes] = _free_bytes(dev) >= RECORDS_OF_FREE * nbytes
             if not self._roomy[nbytes]:
                 return None
         try:
@@ -160,14 +158,8 @@ class AdjointIntegrator:
             records = self._records(prep, n_runs, record, dev)
             count = torch.zeros((n_runs,), device=dev, dtype=torch.int32)
             ckpt = tape = steps = None
-            params_kept, tol_kept = params_t, tol_t
             if records is not None:
                 steps = torch.empty((n_runs,), device=dev, dtype=torch.int32)
-                # checkpoints hold each run's parameters and tolerance scale,
-                # records do not: the reverse sweep reads copies, whatever the
-                # caller writes to its own tensors meanwhile
-                params_kept = params_t.clone()
-                tol_kept = None if tol_t is None else tol_t.clone()
             else:
                 ckpt = torch.empty((n_runs * self.max_ckpts * words,), device=dev, dtype=torch.int32)
                 tape = self._tape_buffers(n_runs, tape_entry, dev) if tape_entry > 0 else None
@@ -180,6 +172,14 @@ class AdjointIntegrator:
         self._set_tape(adj, tape)
         self._set_records(adj, records, steps, n_runs)
         prep["module"].adjoint_launch(args, adj, 0, s.block_size, 0, st.cuda_stream, records is not None)
+        params_kept, tol_kept = params_t, tol_t
+        if records is not None:
+            # checkpoints hold each run's parameters and tolerance scale,
+            # records do not: the reverse sweep reads copies (made behind the
+            # launch), whatever the caller writes to its own tensors meanwhile
+            with torch.cuda.stream(st):
+                params_kept = params_t.clone()
+                tol_kept = None if tol_t is None else tol_t.clone()
         saved = dict(prep=prep, bufs=bufs, inits=inits_t, params=params_kept, tol=tol_kept, ckpt=ckpt, count=count,
                      words=words, record=record, tape=tape, records=records, steps=steps,
                      n_runs=n_runs, duration=duration, settling_time=settling_time, t0=t0, dev=dev, tdtype=tdtype)

@@ -209,31 +209,38 @@ def test_inputs_written_between_forward_and_backward(cuda_device, name, share):
 
 @pytest.mark.gpu
 def test_records_leave_room_for_the_caller(cuda_device, monkeypatch):
-    """Large records need four times their size free (the device's, or unused
-    in torch's pool); the answer stays with the integrator and the size."""
+    """Large records need four times their size besides torch's tensors; the
+    answer stays with the integrator and the size."""
     import torch
     from cubie_b200 import adjoint
     s = _solver("fhn")
     x0, p = (torch.tensor(v.astype(np.float32), device="cuda") for v in _batch("fhn", 64, 3))
     nbytes = 64 * 64 * 64 * 16
-    free = {"device": 0, "pool": 0}
-    asked = []
+    free = []
     monkeypatch.setattr(adjoint, "RECORDS_UNASKED", 0)
-    monkeypatch.setattr(torch.cuda, "mem_get_info", lambda dev=None: (asked.append(1), (free["device"], 1 << 37))[1])
-    monkeypatch.setattr(torch.cuda, "memory_reserved", lambda dev=None: free["pool"] + 1000)
-    monkeypatch.setattr(torch.cuda, "memory_allocated", lambda dev=None: 1000)
-    for device, pool, records in ((4 * nbytes, 0, True), (4 * nbytes - 1, 0, False), (nbytes, 3 * nbytes, True),
-                                  (nbytes, 3 * nbytes - 1, False)):
-        free.update(device=device, pool=pool)
+    monkeypatch.setattr(adjoint, "_free_bytes", lambda dev: free.pop())
+    for room in (4 * nbytes, 4 * nbytes - 1):
+        free.append(room)
         integ = adjoint.AdjointIntegrator(s)
-        asked.clear()
         for _ in range(3):
             _, _, saved = integ.forward(x0, p, 2.0)
-            assert (saved["records"] is not None) == records
-        assert len(asked) == 1
+            assert (saved["records"] is not None) == (room == 4 * nbytes)
+        assert not free
     monkeypatch.setattr(adjoint, "RECORDS_UNASKED", nbytes)          # small records are not asked for
     _, _, saved = adjoint.AdjointIntegrator(s).forward(x0, p, 2.0)
-    assert saved["records"] is not None and len(asked) == 1
+    assert saved["records"] is not None
+
+
+@pytest.mark.gpu
+def test_free_bytes_follow_the_tensors(cuda_device):
+    import torch
+    from cubie_b200.adjoint import _free_bytes
+    total = torch.cuda.get_device_properties(0).total_memory
+    before = _free_bytes(0)
+    big = torch.empty((1 << 28,), dtype=torch.uint8, device="cuda")
+    assert before - _free_bytes(0) == big.numel() and before <= total
+    del big
+    assert _free_bytes(0) == before
 
 
 @pytest.mark.gpu
