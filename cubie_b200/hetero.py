@@ -57,7 +57,9 @@ def _per_run(values, n: int, name: str, dev):
     if values is None:
         return None
     torch = _torch()
-    t = torch.as_tensor(values).to(device=dev, dtype=torch.float64).reshape(-1).contiguous()
+    t = torch.as_tensor(values).to(device=dev, dtype=torch.float64)
+    if t.dim() != 1 or not t.is_contiguous():
+        t = t.reshape(-1).contiguous()
     if t.numel() != n:
         raise ValueError(f"{name} must have one entry per run")
     return t
@@ -239,14 +241,20 @@ class HeteroLaunch:
         self.owner, self.batches, self.module, self.hargs = owner, batches, module, hargs
         self.work, self.preps, self.bufs, self._keep, self.grid = work, preps, bufs, keep, grid
 
+    def _clear(self) -> None:
+        self.work.zero_()
+        for bf in self.bufs:
+            bf["totals"].zero_()
+
     def launch(self, stream, hargs=None) -> None:
         """Zero the run counters and iteration totals, then launch, on
         ``stream`` (capturable: no allocation, no synchronisation)."""
         torch = _torch()
-        with torch.cuda.stream(stream):
-            self.work.zero_()
-            for bf in self.bufs:
-                bf["totals"].zero_()
+        if stream == torch.cuda.current_stream(self.work.device):
+            self._clear()
+        else:
+            with torch.cuda.stream(stream):
+                self._clear()
         self.module.launch_hetero(hargs or self.hargs, self.owner.block_size, self.grid, stream.cuda_stream)
 
     def timed_launch(self, stream=None) -> float:

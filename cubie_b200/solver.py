@@ -604,10 +604,14 @@ class Solver:
     def _settings(self) -> Tuple:
         """The settings of now, as a key: a prepared launch is used again
         while they are the ones it was prepared under."""
+        vectors = _VECTOR_SETTINGS(self)
+        try:
+            vectors = tuple(map(np.ndarray.tobytes, vectors))
+        except TypeError:                   # assigned as lists
+            vectors = tuple(np.asarray(v, dtype=np.float64).tobytes() for v in vectors)
         return (_SCALAR_SETTINGS(self), id(self.tableau), tuple(self.flags.values()),
                 tuple(self._user_timing.values()), tuple(self.summary_plan.metrics),
-                *(tuple(v) for v in _LIST_SETTINGS(self)),
-                *(np.asarray(v, dtype=np.float64).tobytes() for v in _VECTOR_SETTINGS(self)))
+                *map(tuple, _LIST_SETTINGS(self)), vectors)
 
     def prepare(self, duration: float, settling_time: float = 0.0, t0: float = 0.0,
                 interp=None, durations=None, load: bool = True) -> Dict[str, Any]:
@@ -777,9 +781,11 @@ class Solver:
             return None
         if tol_t is None:
             return dur_t, None
-        if tol_t.device != dur_t.device or tuple(tol_t.shape) not in ((n,), (1,), ()):
+        if tol_t.device != dur_t.device or tol_t.dim() > 1 or tol_t.numel() not in (n, 1):
             return None
-        return dur_t, tol_t.to(torch.float64).expand(n).contiguous()
+        if tol_t.numel() != n or tol_t.dtype != torch.float64 or not tol_t.is_contiguous():
+            tol_t = tol_t.to(torch.float64).expand(n).contiguous()
+        return dur_t, tol_t
 
     def run_order(self, dur_t, tol_t=None):
         """Claim order of a persistent launch: with per-run horizons and
