@@ -81,12 +81,11 @@ def _units(a, b, tol):
 
 # FP64: the ring of 128 exceeds the lanes' registers (832 bytes) and run in
 # the shared-memory form although the generator offers the other one
-@pytest.mark.parametrize("name", list(MODELS))
-@pytest.mark.parametrize("placement", ["local", "shared", "registers"])
+@pytest.mark.parametrize("name,placement", [
+    *((name, placement) for name in MODELS for placement in ("local", "shared", "registers") if name != "ring128"),
+    ("ring128", "local")])
 def test_forms_match_the_oracle(cuda_device, name, placement):
     from oracle import OracleSystem, integrate
-    if placement != "local" and name == "ring128":
-        pytest.skip("one placement of the largest system")
     model, n, T, tol = MODELS[name], 5, 0.5, 1e-8
     x0, p = _model_inputs(name, n)
     some = [0, 1, 31, 32, 33, x0.shape[0] - 1]       # ends of slots, a saved and summarised subset
