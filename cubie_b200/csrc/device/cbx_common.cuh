@@ -107,9 +107,9 @@ __device__ __forceinline__ double exp2_t(double a) { return exp2(a); }
 // reciprocal is the division's value.  For every term and tolerance of the
 // norms it has the division's bits (tests/test_ratio_gpu.py); tolerances below
 // 2^-1022 count as zero and those above 2^1021 as infinite.  Divisions were
-// what the FP64 norms cost: Tsit5, 50,021 Lorenz runs 939 -> 884 us; ROS3P,
-// 20,001 Van der Pol runs 1.85 -> 1.61 ms; Radau IIA5 with GMRES, 10,001 runs
-// 7.04 -> 6.09 ms.
+// what the FP64 norms cost: Tsit5, 50,021 Lorenz runs 949 -> 908 us; ROS3P,
+// 20,001 Van der Pol runs 1.85 -> 1.62 ms; Radau IIA5 with GMRES, 10,001 runs
+// 7.04 -> 6.13 ms.
 __device__ __forceinline__ float ratio_t(float e, float tol) { return e / tol; }
 __device__ __forceinline__ double ratio_t(double e, double tol) {
 #ifdef CBX_HOST_EMULATION
@@ -134,7 +134,9 @@ __device__ __forceinline__ double pow_t(double a, double b) { return pow(a, b); 
 // [1, 2): b k is formed exactly for b rounded to a multiple of 2^-40, its
 // integer part becomes the result's exponent, and log2 m, the remainder of b
 // and the fraction are a few units at most, so the result is about as close as
-// pow's (tests/test_gain_powers_gpu.py) at half its instructions.  Finite
+// pow's (tests/test_gain_powers_gpu.py) at half its instructions: with pow and
+// the division in the norms Tsit5 on 50,021 Lorenz runs took 1,233 us, ROS3P on
+// 20,001 Van der Pol runs 2,280, now 917 and 1,641.  Finite
 // a >= 0 (the controllers map other norms to 1e16); zero and subnormal a count
 // as 2^-1023 and infinity as 2^1024, whose powers lie beyond a gain's clamp.
 struct Log2Parts {
@@ -167,8 +169,8 @@ __device__ __forceinline__ double pow_t(double a, double b) {
 #endif
 
 // c a^x b^y for a, b > 0.  In FP64 on the device one exponential serves both
-// powers (Tsit5 FP64, 50,021 Lorenz runs: 996 -> 942 us); in FP32 the two
-// approximate powers side by side have the shorter chain.
+// powers; in FP32 the two approximate powers side by side have the shorter
+// chain.
 __device__ __forceinline__ float scaled_powers(float c, float a, float x, float b, float y) {
     return c * pow_t(a, x) * pow_t(b, y);
 }
