@@ -97,7 +97,7 @@ EXPORTED = (
     "cbx_module_load", "cbx_module_create", "cbx_module_destroy", "cbx_kernel_info",
     "cbx_occupancy", "cbx_solve", "cbx_device_info", "cbx_fp32_peak_probe", "cbx_flush_l2",
     "cbx_solve_noalloc", "cbx_adjoint_info", "cbx_adjoint_tape_bytes", "cbx_adjoint_launch", "cbx_solve_hetero",
-    "cbx_claim_order", "cbx_adjoint_launch_records", "cbx_adjoint_lanes",
+    "cbx_claim_order", "cbx_adjoint_launch_records", "cbx_adjoint_lanes", "cbx_persistent_blocks",
 )
 
 _lib = None
@@ -146,6 +146,8 @@ def lib():
         L.cbx_occupancy.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.c_int, ctypes.POINTER(ctypes.c_int)]
         L.cbx_solve.argtypes = [ctypes.c_void_p, ctypes.POINTER(SolveArgs), ctypes.c_int, ctypes.c_int,
                                 ctypes.c_int, ctypes.c_void_p]
+        L.cbx_persistent_blocks.argtypes = [ctypes.c_longlong, ctypes.c_int, ctypes.c_int, ctypes.c_longlong,
+                                            ctypes.c_int, ctypes.POINTER(ctypes.c_longlong)]
         L.cbx_device_info.argtypes = [ctypes.c_int] + [ctypes.POINTER(ctypes.c_int)] * 3
         L.cbx_fp32_peak_probe.argtypes = [ctypes.c_int, ctypes.POINTER(ctypes.c_double),
                                           ctypes.POINTER(ctypes.c_float)]
@@ -299,6 +301,14 @@ def device_info(device: int = 0) -> dict:
     sm, a, b = ctypes.c_int(), ctypes.c_int(), ctypes.c_int()
     _check(lib().cbx_device_info(device, ctypes.byref(sm), ctypes.byref(a), ctypes.byref(b)), "cbx_device_info")
     return dict(sm_count=sm.value, cc=(a.value, b.value))
+
+
+def persistent_blocks(resident: int, sm_count: int, block: int, runs: int, local_bytes: int) -> int:
+    """Blocks a persistent launch takes with grid = 0 (no device needed)."""
+    v = ctypes.c_longlong()
+    _check(lib().cbx_persistent_blocks(resident, sm_count, block, runs, local_bytes, ctypes.byref(v)),
+           "cbx_persistent_blocks")
+    return v.value
 
 
 def fp32_peak(device: int = 0) -> float:

@@ -340,6 +340,43 @@ int cbx_occupancy(cbx_module* module, int kernel, int block, int* blocks_per_sm)
 }  // extern "C"
 
 namespace {
+// Blocks of a persistent launch: what the runs need, at most the resident ones.
+//
+// A batch that fills less than one warp per scheduler is spread over that many
+// (the kernel then uses as many lanes of each warp as the runs need): its time
+// is the slowest lane's chain of dependent instructions, a warp's lanes wait
+// for one another where they branch apart, and the other schedulers are idle.
+// 128-thread blocks, packed against one block per SM: Lorenz, 96 runs 75 -> 63
+// us, 4,096 runs saving rows 224 -> 191; Van der Pol, 5,001 runs with GMRES
+// 2.87 -> 2.71 ms, 10,001 under Radau IIA 3.02 -> 2.85.  (That reaches every SM
+// with blocks of at most 128 threads; larger blocks are as many warps on fewer
+// SMs.)  From two warps per scheduler on the warps slow each other (the 4,096
+// runs: 205 us at two, 237 at three).
+//
+// Kernels that keep arrays in local memory are those of larger systems, with
+// hundreds of kilobytes of unrolled code: what they wait for is instructions,
+// and every further warp fetches all of them.  They are spread only while each
+// run has a warp to itself.  12 states, packed against spread: ROS3P with
+// GMRES, 300 runs FP64 4.59 -> 3.97 ms, but 3,000 runs FP32 1.53 -> 2.17, FP64
+// 4.67 -> 5.44, 9,000 runs 1.98 -> 2.85 and 5.30 -> 6.43; SDIRK4 with BiCGSTAB,
+// FP32, 9,000 runs 0.95 -> 1.12; direct ROS3P gains to 9,000 runs (2.59 -> 2.32)
+// and loses at 16,000 (2.58 -> 2.77).  (A few bytes are one spilled vector of a
+// small kernel: Kvaerno 5 with GMRES, 1,000 Van der Pol runs 1.32 -> 0.93.)
+long long persistent_blocks(long long resident, int sm_count, int block, long long runs, int local) {
+    long long blocks = (runs + block - 1) / block;
+    const long long spread = (long long)sm_count * 128 / block;
+    if (local <= 64 || runs <= spread * (block / 32)) {
+        const long long least = spread < runs ? spread : runs;
+        if (blocks < least) blocks = least;
+    }
+    return blocks < resident ? blocks : resident;
+}
+
+int local_bytes(CUfunction f) {
+    int v = 0;
+    return g_drv.cuFuncGetAttribute(&v, CU_FUNC_ATTRIBUTE_LOCAL_SIZE_BYTES, f) == CUDA_SUCCESS ? v : 0;
+}
+
 // Argument checks of cbx_solve; ``need_counter`` = false for callers that
 // supply the work counter themselves.
 int validate_solve(const cbx_module* module, const cbx_solve_args* args, int kernel, int block, bool need_counter) {
@@ -384,24 +421,8 @@ int cbx_solve(cbx_module* module, const cbx_solve_args* args, int kernel, int bl
             g = (long long)per_sm * module->sm_count;
             const long long runs_per_block = kernel == CBX_KERNEL_WARP ? block / 32 : block;
             long long needed = (args->n_runs + runs_per_block - 1) / runs_per_block;
-            if (kernel == CBX_KERNEL_PERSISTENT) {
-                // A batch that fills less than one warp per scheduler is
-                // spread over that many (the kernel then uses as many lanes
-                // of each warp as the runs need): its time is the slowest
-                // lane's chain of dependent instructions, a warp's lanes
-                // wait for one another where they branch apart, and the other
-                // schedulers are idle.  128-thread blocks, packed against one
-                // block per SM: Lorenz, 96 runs 75 -> 63 us, 4,096 runs
-                // saving rows 224 -> 191; Van der Pol, 5,001 runs with GMRES
-                // 2.87 -> 2.71 ms, 10,001 under Radau IIA 3.02 -> 2.85.  (That
-                // reaches every SM with blocks of at most 128 threads; larger
-                // blocks are as many warps on fewer SMs.)  From
-                // two warps per scheduler on the warps slow each other (the
-                // 4,096 runs: 205 us at two, 237 at three).
-                const long long spread = (long long)module->sm_count * 128 / block;
-                const long long least = spread < args->n_runs ? spread : args->n_runs;
-                if (needed < least) needed = least;
-            }
+            if (kernel == CBX_KERNEL_PERSISTENT)
+                needed = persistent_blocks(g, module->sm_count, block, args->n_runs, local_bytes(module->fn[kernel]));
             if (g > needed) g = needed;
         }
     }
@@ -414,6 +435,13 @@ int cbx_solve(cbx_module* module, const cbx_solve_args* args, int kernel, int bl
     return check_cu(g_drv.cuLaunchKernel(module->fn[kernel], (unsigned)g, 1, 1, (unsigned)block, 1, 1, smem,
                                    static_cast<CUstream>(stream), params, nullptr),
                     "cuLaunchKernel");
+}
+
+int cbx_persistent_blocks(long long resident, int sm_count, int block, long long runs, int local, long long* blocks) {
+    if (resident < 1 || sm_count < 1 || block <= 0 || block > 1024 || (block % 32) != 0 || runs < 0 || local < 0 || !blocks)
+        return fail(CBX_ERR_ARGUMENT, "bad launch shape");
+    *blocks = persistent_blocks(resident, sm_count, block, runs, local);
+    return CBX_OK;
 }
 
 int cbx_device_info(int device, int* sm_count, int* cc_major, int* cc_minor) {
@@ -579,14 +607,9 @@ int adjoint_launch(cbx_module* module, const cbx_solve_args* args, const cbx_adj
             per_sm = 1;
         g = (long long)per_sm * module->sm_count;
         long long needed = (args->n_runs + block - 1) / block;
-        if (records) {
-            // small batches spread as in cbx_solve (forward + backward, packed
-            // against spread: 5,000 FitzHugh-Nagumo runs 577 -> 478 us, 8,191
-            // Van der Pol runs under ROS3P 847 -> 813)
-            const long long spread = (long long)module->sm_count * 128 / block;
-            const long long least = spread < args->n_runs ? spread : args->n_runs;
-            if (needed < least) needed = least;
-        }
+        // (forward + backward, packed against spread: 5,000 FitzHugh-Nagumo runs
+        // 577 -> 478 us, 8,191 Van der Pol runs under ROS3P 847 -> 813)
+        if (records) needed = persistent_blocks(g, module->sm_count, block, args->n_runs, local_bytes(f));
         if (g > needed) g = needed;
     }
     if (g > 2147483647LL) return fail(CBX_ERR_ARGUMENT, "grid too large");

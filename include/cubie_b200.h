@@ -76,6 +76,11 @@ int cbx_kernel_info(cbx_module* module, int kernel, int* registers, int* local_b
 /* Resident blocks per SM for ``block`` threads. */
 int cbx_occupancy(cbx_module* module, int kernel, int block, int* blocks_per_sm);
 
+/* Blocks that a persistent launch of ``runs`` runs takes with grid = 0, for a
+ * kernel of which ``resident`` blocks fit the device's ``sm_count`` SMs and
+ * which keeps ``local`` bytes of local memory a thread (no device needed). */
+int cbx_persistent_blocks(long long resident, int sm_count, int block, long long runs, int local, long long* blocks);
+
 /* Launch the integration kernel: the replacement for the reference's
  * kernel launch (BatchSolverKernel.py:741-762).  ``args`` holds caller
  * device pointers (layouts in cbx_args.h).  grid = 0 picks
