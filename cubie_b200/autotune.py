@@ -60,7 +60,7 @@ def default_candidates(solver) -> List[Tuple]:
             return list(WARP_CANDIDATES)
         return [(b, 0, solver.scratch_placement, r) for b in (128, 64) for r in (0, 168)] + [
             (128, 1, solver.scratch_placement, 0)]
-    if bounds_registers(solver.tableau.kind, solver.linear_correction_type):
+    if bounds_registers(solver.tableau.kind, solver.linear_correction_type, solver.system.num_states):
         return [*RULE_CANDIDATES, *DEFAULT_CANDIDATES]
     return list(DEFAULT_CANDIDATES)
 

@@ -368,30 +368,35 @@ def family_block(system: SymbolicODE, spec: KernelSpec, gen: GeneratedSystem, ns
     return lines
 
 
-def bounds_registers(kind: str, linear_correction_type: str) -> bool:
+def bounds_registers(kind: str, linear_correction_type: str, n_states: int) -> bool:
     """Whether ``thread_min_blocks`` bounds the step's registers."""
-    return kind == FIRK or (kind == ROSENBROCK and linear_correction_type == "direct")
+    return kind == FIRK or (kind == ROSENBROCK and linear_correction_type == "direct" and n_states <= 4)
 
 
-def thread_min_blocks(spec: KernelSpec) -> int:
+def thread_min_blocks(spec: KernelSpec, n_states: int) -> int:
     """Minimum of resident blocks per SM in the kernels' launch bounds (0:
     none): the caller's, or where the caller named neither it nor a register
-    cap, 256 threads' worth for fully implicit steps and direct Rosenbrock
-    steps.
+    cap, 256 threads' worth for fully implicit steps and for direct Rosenbrock
+    steps of up to four states.
 
     Without one the compiler holds these kernels to the registers of a higher
     occupancy than they profit from; asked for two 128-thread blocks it spends
     more of them and the step's chain gets shorter.  Measured, none against
     two: Radau IIA5 direct, 60,001 Van der Pol runs 5.01 -> 4.15 ms, with GMRES,
     65,536 runs 4.37 -> 4.07; ROS3P direct FP64, 100,001 runs 3.43 -> 3.06, FP32
-    with FP64 control, 524,288 runs 2.70 -> 2.65.  Explicit steps and Rosenbrock
+    with FP64 control, 524,288 runs 2.70 -> 2.65.  Four states, 40,000 runs: ROS3P
+    FP32 0.156 -> 0.151, FP64 0.660 -> 0.649, RODAS3P mixed 0.475 -> 0.455; Radau
+    IIA5 direct FP32 7.39 -> 6.59, and with GMRES at eight FP64 10.7 -> 9.1.
+    Larger direct Rosenbrock steps fill the registers anyway and only come out
+    otherwise: ROS3P FP32 of eight states 0.58 -> 0.64, twelve, 100,000 runs
+    12.1 -> 13.4 (mixed 26.9 -> 30.3).  Explicit steps and Rosenbrock
     or DIRK steps with a Krylov solver lose or stay (Tsit5 FP64 2.19 -> 2.30,
     ROS3P with GMRES 4.31 -> 4.44, SDIRK4 0.98 -> 0.99); more blocks spill."""
     if int(spec.min_blocks_per_sm):
         return int(spec.min_blocks_per_sm) if int(spec.min_blocks_per_sm) > 1 else 0
     if spec.max_registers:
         return 0
-    if bounds_registers(spec.tableau.kind, spec.linear_correction_type):
+    if bounds_registers(spec.tableau.kind, spec.linear_correction_type, n_states):
         return max(1, 256 // int(spec.block_size))
     return 0
 
@@ -406,7 +411,7 @@ def generate_kernel(system: SymbolicODE, spec: KernelSpec, gen: Optional[Generat
     if spec.layout == "warp":
         return _generate_warp_kernel(system, spec, gen, warp_code)
     lines = ["// generated by cubie_b200.kernelgen; do not edit"]
-    min_blocks = thread_min_blocks(spec)
+    min_blocks = thread_min_blocks(spec, system.num_states)
     if min_blocks:
         lines.append(f"#define CBX_LAUNCH_BOUNDS(CFG) __launch_bounds__(CFG::BLOCK, {min_blocks})")
     lines += DEVICE_INCLUDES
@@ -445,8 +450,8 @@ def generate_hetero_kernel(families: Sequence[Tuple[SymbolicODE, KernelSpec, Gen
     # 0.91 -> 0.86; 200,000 Lorenz with 2,000 Van der Pol 0.77 -> 0.76; 150,000
     # Lorenz with 5,000 Radau IIA5 runs 24.3 -> 21.3; FP64 Lorenz, 100,000,
     # with 2,000 Van der Pol 1.70, 1.70 ms
-    min_blocks = max(thread_min_blocks(replace(spec, block_size=block, min_blocks_per_sm=0, max_registers=0))
-                     for _, spec, _ in families)
+    min_blocks = max(thread_min_blocks(replace(spec, block_size=block, min_blocks_per_sm=0, max_registers=0),
+                                       system.num_states) for system, spec, _ in families)
     if min_blocks:
         lines.append(f"#define CBX_HETERO_BOUNDS(BLOCK) __launch_bounds__(BLOCK, {min_blocks})")
     lines += DEVICE_INCLUDES

@@ -39,6 +39,23 @@ def test_callers_choice_goes_before_the_rule(algorithm, linear, rule):
     assert _minimum(_vdp(max_registers=64, min_blocks_per_sm=3, **kw)) == 3
 
 
+@pytest.mark.parametrize("algorithm,linear", [("ros3p", "direct"), ("radau", "direct"), ("radau", "gmres")])
+@pytest.mark.parametrize("n", [3, 4, 5, 8])
+def test_rule_by_states(algorithm, linear, n):
+    """Direct Rosenbrock steps are bounded up to four states, fully implicit
+    ones always."""
+    from cubie_b200 import Solver, create_ODE_system
+    from cubie_b200.autotune import RULE_CANDIDATES, default_candidates
+    if linear == "direct" and algorithm == "radau" and n > 4:
+        linear = "gmres"                     # the operator of a direct solve is too wide
+    sysm = create_ODE_system([f"du{i} = u{(i + 1) % n} - k * u{i}**3" for i in range(n)],
+                             states=[f"u{i}" for i in range(n)], parameters=["k"], precision=np.float32)
+    s = Solver(sysm, algorithm=algorithm, linear_correction_type=linear, output_types=["state"])
+    bounded = algorithm == "radau" or n <= 4
+    assert _minimum(s) == (2 if bounded else None)
+    assert (RULE_CANDIDATES[0] in default_candidates(s)) == bounded
+
+
 def test_warp_layout_takes_the_callers_choice():
     from cubie_b200 import Solver, create_ODE_system
     eqs, states, params, _ = hh_cable(64)
