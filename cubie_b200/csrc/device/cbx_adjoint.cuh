@@ -813,28 +813,25 @@ __device__ __forceinline__ void run_adjoint_backward(const cbx_solve_args a, con
 // that all keep step, whose stores were whole lines, 0.73 -> 0.80 (1.02).  At
 // 40,000 runs pairs gain nothing (1.37, 1.39), and groups of four or eight steps
 // cost the runs that keep step more than they save the others (0.84 and 0.92
-// against 2.90 and 2.96).  Each kernel holds its loop once for either layout.
+// against 2.90 and 2.96).  The host picks the kernels (runtime.cu).
 template <class Cfg, bool PAIRS>
 struct RecordPlace {
     using R = typename Cfg::R;
     static constexpr int F = SegRecord<Cfg>::F;
-    // record j of a run, and the values between records j and j + 1
-    static __device__ __forceinline__ R* at(const cbx_adjoint_args& g, long long run, int j) {
+    // record j of a run, and the values between records j and j + 1 (``wide`` for
+    // every j, or for the odd ones of pairs)
+    static __device__ __forceinline__ R* at(const cbx_adjoint_args& g, long long wide, long long run, int j) {
         R* records = static_cast<R*>(g.seg);
         if constexpr (PAIRS) return records + ((j & ~1) * g.lane_words + 2 * run + (j & 1)) * F;
-        else return records + (j * g.lane_words + run) * F;
+        else return records + run * F + j * wide;
     }
-    static __device__ __forceinline__ long long step(const cbx_adjoint_args& g, int j) {
-        if constexpr (PAIRS) return (j & 1) ? (2 * g.lane_words - 1) * F : F;
-        else return g.lane_words * F;
+    static __device__ __forceinline__ long long wide(const cbx_adjoint_args& g) {
+        return PAIRS ? (2 * g.lane_words - 1) * F : g.lane_words * F;
+    }
+    static __device__ __forceinline__ long long step(long long wide, int j) {
+        return PAIRS && !(j & 1) ? F : wide;
     }
 };
-
-template <class Cfg>
-__device__ __forceinline__ bool records_in_pairs(const cbx_adjoint_args& g) {
-    return SegRecord<Cfg>::F * int(sizeof(typename Cfg::R)) < 32 && g.lane_words > 65536 &&
-           ((g.max_ckpts * g.ckpt_every) & 1) == 0;
-}
 
 template <class Cfg, bool PAIRS>
 struct RecordWriter {
@@ -842,8 +839,8 @@ struct RecordWriter {
     using C = typename Cfg::C;
     using Rec = SegRecord<Cfg>;
     static constexpr bool ACTIVE = true;
-    const cbx_adjoint_args& g;
     R* next;
+    long long wide;
     int count;
     __device__ __forceinline__ void accepted(const Lane<Cfg>& L, C dt_eff, int row) {
         R rec[Rec::F];
@@ -855,27 +852,27 @@ struct RecordWriter {
 #pragma unroll
         for (int k = Rec::H_AT + 1; k < Rec::F; ++k) rec[k] = R(0);
         Rec::store(next, rec);
-        next += RecordPlace<Cfg, PAIRS>::step(g, count);
+        next += RecordPlace<Cfg, PAIRS>::step(wide, count);
         ++count;
     }
 };
 
 template <class Cfg, bool PAIRS>
-__device__ __forceinline__ void forward_records(const cbx_solve_args& a, const cbx_adjoint_args& g) {
+__device__ __forceinline__ void run_adjoint_forward_records(const cbx_solve_args a, const cbx_adjoint_args g) {
     using R = typename Cfg::R;
     __shared__ BlockTotals bt;
     totals_begin(&bt);
     Lane<Cfg> L;
     bool active = false, exhausted = !lane_in_use(a.n_runs);
     const int cap = g.max_ckpts * g.ckpt_every;
-    RecordWriter<Cfg, PAIRS> rec{g, nullptr, 0};
+    RecordWriter<Cfg, PAIRS> rec{nullptr, RecordPlace<Cfg, PAIRS>::wide(g), 0};
     while (true) {
         if (!active && !exhausted) {
             const long long run = claim_run(a.work_counter);
             if (run < a.n_runs) {
                 lane_begin<Cfg>(L, a, run);
                 active = true;
-                rec.next = RecordPlace<Cfg, PAIRS>::at(g, run, 0);
+                rec.next = RecordPlace<Cfg, PAIRS>::at(g, rec.wide, run, 0);
                 rec.count = 0;
             } else {
                 exhausted = true;
@@ -906,13 +903,14 @@ __device__ __forceinline__ void forward_records(const cbx_solve_args& a, const c
 // Reverse sweep over the records: every lane walks its own run backwards, the
 // next (earlier) record and the next saved row's loss gradient in flight.
 template <class Cfg, bool PAIRS>
-__device__ __forceinline__ void backward_records(const cbx_solve_args& a, const cbx_adjoint_args& g) {
+__device__ __forceinline__ void run_adjoint_backward_records(const cbx_solve_args a, const cbx_adjoint_args g) {
     using R = typename Cfg::R;
     using C = typename Cfg::C;
     using Adj = StepAdjoint<Cfg, Cfg::ALGO>;
     using Rec = SegRecord<Cfg>;
     constexpr int N = Cfg::N, NP = Cfg::NP, F = Rec::F, NPP = NP > 0 ? NP : 1;
     const long long s = a.run_stride;
+    const long long wide = RecordPlace<Cfg, PAIRS>::wide(g);
     const R* params = static_cast<const R*>(a.params);
     R lam[N], p[NPP], nxt[F];
     C pbar[NPP];
@@ -938,7 +936,7 @@ __device__ __forceinline__ void backward_records(const cbx_solve_args& a, const 
                 j = g.step_count[run] - 1;
                 rows_end = g.ckpt_count[run];
                 if (j >= 0) {
-                    rec_at = RecordPlace<Cfg, PAIRS>::at(g, run, j);
+                    rec_at = RecordPlace<Cfg, PAIRS>::at(g, wide, run, j);
                     Rec::load(rec_at, nxt);
                     row_next.load(a, g, rows_end - 1, run);
                 }
@@ -952,7 +950,7 @@ __device__ __forceinline__ void backward_records(const cbx_solve_args& a, const 
 #pragma unroll
             for (int k = 0; k < F; ++k) rec_j[k] = nxt[k];
             if (j > 0) {
-                rec_at -= RecordPlace<Cfg, PAIRS>::step(g, j - 1);
+                rec_at -= RecordPlace<Cfg, PAIRS>::step(wide, j - 1);
                 Rec::load(rec_at, nxt);
             }
             const R hs = rec_j[Rec::H_AT];
@@ -983,17 +981,6 @@ __device__ __forceinline__ void backward_records(const cbx_solve_args& a, const 
     }
 }
 
-template <class Cfg>
-__device__ __forceinline__ void run_adjoint_forward_records(const cbx_solve_args& a, const cbx_adjoint_args& g) {
-    if (records_in_pairs<Cfg>(g)) forward_records<Cfg, true>(a, g);
-    else forward_records<Cfg, false>(a, g);
-}
-template <class Cfg>
-__device__ __forceinline__ void run_adjoint_backward_records(const cbx_solve_args& a, const cbx_adjoint_args& g) {
-    if (records_in_pairs<Cfg>(g)) backward_records<Cfg, true>(a, g);
-    else backward_records<Cfg, false>(a, g);
-}
-
 }  // namespace cbx
 
 #define CBX_DEFINE_ADJOINT_KERNELS(CFG)                                                              \
@@ -1010,9 +997,17 @@ __device__ __forceinline__ void run_adjoint_backward_records(const cbx_solve_arg
     }                                                                                                 \
     extern "C" __global__ void CBX_LAUNCH_BOUNDS(CFG) cbx_adjoint_forward_records(cbx_solve_args a,    \
                                                                                  cbx_adjoint_args g) { \
-        cbx::run_adjoint_forward_records<CFG>(a, g);                                                  \
+        cbx::run_adjoint_forward_records<CFG, false>(a, g);                                           \
     }                                                                                                 \
     extern "C" __global__ void CBX_LAUNCH_BOUNDS(CFG) cbx_adjoint_backward_records(cbx_solve_args a,   \
                                                                                   cbx_adjoint_args g) { \
-        cbx::run_adjoint_backward_records<CFG>(a, g);                                                 \
+        cbx::run_adjoint_backward_records<CFG, false>(a, g);                                          \
+    }                                                                                                 \
+    extern "C" __global__ void CBX_LAUNCH_BOUNDS(CFG) cbx_adjoint_forward_pairs(cbx_solve_args a,      \
+                                                                               cbx_adjoint_args g) {  \
+        cbx::run_adjoint_forward_records<CFG, true>(a, g);                                            \
+    }                                                                                                 \
+    extern "C" __global__ void CBX_LAUNCH_BOUNDS(CFG) cbx_adjoint_backward_pairs(cbx_solve_args a,     \
+                                                                                cbx_adjoint_args g) { \
+        cbx::run_adjoint_backward_records<CFG, true>(a, g);                                           \
     }

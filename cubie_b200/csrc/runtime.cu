@@ -29,7 +29,7 @@ struct cbx_module {
     int sm_count;
     // discrete-adjoint kernels, resolved on first use (modules generated
     // without them have neither)
-    CUfunction adj[4];  // forward, backward, and both again in the record form
+    CUfunction adj[6];  // forward, backward, and both again in the record form, by steps and by pairs
     size_t lane_bytes;
     size_t record_bytes;
     size_t tape_bytes;
@@ -523,9 +523,10 @@ int resolve_adjoint(cbx_module* m) {
     size_t rbytes = 0;
     if (g_drv.cuModuleGetGlobal(&probe2, &rbytes, m->module, "cbx_seg_record_probe") != CUDA_SUCCESS)
         return fail(CBX_ERR_ARGUMENT, "module was generated without the adjoint kernels");
-    const char* names[4] = {"cbx_adjoint_forward", "cbx_adjoint_backward", "cbx_adjoint_forward_records",
-                            "cbx_adjoint_backward_records"};
-    for (int k = 0; k < 4; ++k) {
+    const char* names[6] = {"cbx_adjoint_forward", "cbx_adjoint_backward", "cbx_adjoint_forward_records",
+                            "cbx_adjoint_backward_records", "cbx_adjoint_forward_pairs",
+                            "cbx_adjoint_backward_pairs"};
+    for (int k = 0; k < 6; ++k) {
         int rc = check_cu(g_drv.cuModuleGetFunction(&m->adj[k], m->module, names[k]), names[k]);
         if (rc) return rc;
     }
@@ -599,7 +600,11 @@ int adjoint_launch(cbx_module* module, const cbx_solve_args* args, const cbx_adj
         return fail(CBX_ERR_ARGUMENT, "lane_words (%lld) is smaller than the module's lane image (%zu bytes)",
                     adj->lane_words, module->lane_bytes);
     if (args->n_runs == 0) return CBX_OK;
-    CUfunction f = module->adj[phase + (records ? 2 : 0)];
+    // record layout: pairs of steps above 65,536 runs, where a record is half a
+    // sector (cbx_adjoint.cuh, RecordPlace)
+    const bool pairs = records && module->record_bytes < 32 && adj->lane_words > 65536 &&
+                       (((long long)adj->ckpt_every * adj->max_ckpts) & 1) == 0;
+    CUfunction f = module->adj[phase + (pairs ? 4 : (records ? 2 : 0))];
     long long g = grid;
     if (g <= 0) {
         int per_sm = 0;
@@ -638,7 +643,7 @@ extern "C" int cbx_adjoint_lanes(cbx_module* module, int block, long long* lanes
     if (!rc) rc = resolve_adjoint(module);
     if (rc) return rc;
     *lanes = 0;
-    for (int k = 2; k < 4; ++k) {
+    for (int k = 2; k < 6; ++k) {
         int per_sm = 0;
         rc = check_cu(g_drv.cuOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, module->adj[k], block, 0),
                       "cuOccupancyMaxActiveBlocksPerMultiprocessor");

@@ -157,7 +157,7 @@ int cbx_adjoint_launch(cbx_module* module, const cbx_solve_args* args, const cbx
 int cbx_adjoint_launch_records(cbx_module* module, const cbx_solve_args* args, const cbx_adjoint_args* adj,
                                int phase, int block, int grid, void* stream);
 
-/* Runs that both kernels of the record form hold at once, a lane each, at this
+/* Runs that every kernel of the record form holds at once, a lane each, at this
  * block size. */
 int cbx_adjoint_lanes(cbx_module* module, int block, long long* lanes);
 

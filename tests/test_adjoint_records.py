@@ -22,7 +22,9 @@ extern "C" void emu_records(cbx_solve_args* a, cbx_adjoint_args* g, int phase, i
     for (int t = 0; t < block; ++t) {
         threadIdx = {(unsigned)t, 0, 0};
         if (phase == 0) cbx_adjoint_forward_records(*a, *g);
-        else cbx_adjoint_backward_records(*a, *g);
+        else if (phase == 1) cbx_adjoint_backward_records(*a, *g);
+        else if (phase == 2) cbx_adjoint_forward_pairs(*a, *g);
+        else cbx_adjoint_backward_pairs(*a, *g);
     }
 }
 """
@@ -47,7 +49,7 @@ def _batch(name, n, seed=0):
     return np.stack([rng.uniform(1, 2, n), rng.uniform(-1, 1, n)]), rng.uniform(0.5, 3.0, (1, n))
 
 
-def _emulated_against_replay(name, every, ckpts, lanes=None):
+def _emulated_against_replay(name, every, ckpts, pairs=False):
     """Both forms in emulation: the same bits; returns (steps, statuses)."""
     from emu import compile_emulated, run_emulated_adjoint
     from cubie_b200 import _native
@@ -58,7 +60,7 @@ def _emulated_against_replay(name, every, ckpts, lanes=None):
     prep = s.prepare(T, 0.0, 0.0, None, None, load=False)
     lib = compile_emulated(prep["gen"].source + DRIVER)
     n, cap = x0.shape[1], every * ckpts
-    lanes = lanes or n
+    lanes = n + 3 if pairs else n
     x, q = np.ascontiguousarray(x0, np.float32), np.ascontiguousarray(p, np.float32)
     out = dict(state=np.zeros_like(state), status=np.zeros_like(status), work=np.zeros(2, np.uint64),
                seg=np.full(lanes * cap * int(lib.emu_record_bytes()) // 8 + 2, np.nan), count=np.zeros(n, np.int32),
@@ -75,9 +77,9 @@ def _emulated_against_replay(name, every, ckpts, lanes=None):
     g.ckpt_every, g.max_ckpts = every, ckpts
     g.lane_words = lanes
     g.grad_state, g.grad_inits, g.grad_params = grad.ctypes.data, out["gi"].ctypes.data, out["gp"].ctypes.data
-    lib.emu_records(ctypes.byref(a), ctypes.byref(g), 0, 32)
+    lib.emu_records(ctypes.byref(a), ctypes.byref(g), 2 if pairs else 0, 32)
     out["work"][:] = 0
-    lib.emu_records(ctypes.byref(a), ctypes.byref(g), 1, 32)
+    lib.emu_records(ctypes.byref(a), ctypes.byref(g), 3 if pairs else 1, 32)
     # one compiler, no contraction: the same bits
     np.testing.assert_array_equal(out["state"], state)
     np.testing.assert_array_equal(out["status"], status)
@@ -93,12 +95,12 @@ def test_emulated_records_equal_replay(name):
     assert steps.min() > 2 * 4
 
 
-# records of more than 65,536 lanes lie in pairs of steps where the limit of
-# steps is even; runs that stop at the limit and runs that end before it
+# records in pairs of steps (an even limit of steps); runs that stop at the
+# limit and runs that end before it
 @pytest.mark.parametrize("name", ["fhn", "vdp"])
-@pytest.mark.parametrize("every,ckpts", [(4, 32), (3, 5), (1, 2), (7, 2)])
+@pytest.mark.parametrize("every,ckpts", [(4, 32), (3, 4), (1, 2), (7, 2)])
 def test_emulated_pairs_equal_replay(name, every, ckpts):
-    steps, status = _emulated_against_replay(name, every, ckpts, lanes=65537)
+    steps, status = _emulated_against_replay(name, every, ckpts, pairs=True)
     if every * ckpts <= 15:
         assert np.all(steps == every * ckpts) and np.all(status == 32)
     else:
