@@ -353,19 +353,20 @@ namespace {
 // SMs.)  From two warps per scheduler on the warps slow each other (the 4,096
 // runs: 205 us at two, 237 at three).
 //
-// Kernels that keep arrays in local memory are those of larger systems, with
-// hundreds of kilobytes of unrolled code: what they wait for is instructions,
-// and every further warp fetches all of them.  They are spread only while each
-// run has a warp to itself.  12 states, packed against spread: ROS3P with
-// GMRES, 300 runs FP64 4.59 -> 3.97 ms, but 3,000 runs FP32 1.53 -> 2.17, FP64
-// 4.67 -> 5.44, 9,000 runs 1.98 -> 2.85 and 5.30 -> 6.43; SDIRK4 with BiCGSTAB,
-// FP32, 9,000 runs 0.95 -> 1.12; direct ROS3P gains to 9,000 runs (2.59 -> 2.32)
-// and loses at 16,000 (2.58 -> 2.77).  (A few bytes are one spilled vector of a
-// small kernel: Kvaerno 5 with GMRES, 1,000 Van der Pol runs 1.32 -> 0.93.)
+// Kernels with more than 256 bytes of local memory a thread are those of larger
+// systems, with hundreds of kilobytes of unrolled code: what they wait for is
+// instructions, and every further warp fetches all of them.  They are spread
+// only while each run has a warp to itself.  12 states, packed against spread:
+// ROS3P with GMRES (312 bytes in FP32, 1,480 in FP64), 300 runs FP64 4.59 -> 3.97
+// ms, but 3,000 runs FP32 1.53 -> 2.17, FP64 4.67 -> 5.44, 9,000 runs 1.98 -> 2.85
+// and 5.30 -> 6.43; direct ROS3P (736) gains to 9,000 runs (2.59 -> 2.32) and
+// loses at 16,000 (2.58 -> 2.77).  Below, local memory is a few spilled vectors:
+// Kvaerno 5 with GMRES (8 bytes), 1,000 Van der Pol runs 1.32 -> 0.93, Radau IIA5
+// with GMRES in FP64 (176), 1,000 runs 4.53 -> 4.06, 9,000 4.51 -> 4.57.
 long long persistent_blocks(long long resident, int sm_count, int block, long long runs, int local) {
     long long blocks = (runs + block - 1) / block;
     const long long spread = (long long)sm_count * 128 / block;
-    if (local <= 64 || runs <= spread * (block / 32)) {
+    if (local <= 256 || runs <= spread * (block / 32)) {
         const long long least = spread < runs ? spread : runs;
         if (blocks < least) blocks = least;
     }

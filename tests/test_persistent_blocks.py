@@ -1,6 +1,6 @@
 """Blocks of a persistent launch: small batches are spread over a warp per
-scheduler, kernels with arrays in local memory only while every run has a
-warp to itself (CPU)."""
+scheduler, kernels with more than 256 bytes of local memory only while every
+run has a warp to itself (CPU)."""
 
 import pytest
 
@@ -15,9 +15,9 @@ def test_blocks_by_runs(block, per_sm):
     for runs in (1, 31, 128, 591, 592, 593, 3000, 9000, 18943, 18944, 18945, 40000, 10 ** 6):
         packed = min(-(-runs // block), resident)
         few = min(max(packed, min(spread, runs)), resident)
-        for local in (0, 8, 64):
+        for local in (0, 8, 256):
             assert persistent_blocks(resident, SMS, block, runs, local) == few
-        for local in (65, 96, 4032):
+        for local in (257, 312, 4032):
             assert persistent_blocks(resident, SMS, block, runs, local) == (few if runs <= warps else packed)
     assert persistent_blocks(resident, SMS, block, 0, 0) == 0
 
