@@ -528,7 +528,12 @@ int resolve_adjoint(cbx_module* m) {
                             "cbx_adjoint_backward_records", "cbx_adjoint_forward_pairs",
                             "cbx_adjoint_backward_pairs"};
     for (int k = 0; k < 6; ++k) {
-        int rc = check_cu(g_drv.cuModuleGetFunction(&m->adj[k], m->module, names[k]), names[k]);
+        const CUresult r = g_drv.cuModuleGetFunction(&m->adj[k], m->module, names[k]);
+        if (k >= 2 && r == CUDA_ERROR_NOT_FOUND) {   // an older module: checkpoints only
+            m->adj[k] = nullptr;
+            continue;
+        }
+        int rc = check_cu(r, names[k]);
         if (rc) return rc;
     }
     // a module without the probe keeps no tape
@@ -604,8 +609,9 @@ int adjoint_launch(cbx_module* module, const cbx_solve_args* args, const cbx_adj
     // record layout: pairs of steps above 65,536 runs, where a record is half a
     // sector (cbx_adjoint.cuh, RecordPlace)
     const bool pairs = records && module->record_bytes < 32 && adj->lane_words > 65536 &&
-                       (((long long)adj->ckpt_every * adj->max_ckpts) & 1) == 0;
+                       (((long long)adj->ckpt_every * adj->max_ckpts) & 1) == 0 && module->adj[4] && module->adj[5];
     CUfunction f = module->adj[phase + (pairs ? 4 : (records ? 2 : 0))];
+    if (!f) return fail(CBX_ERR_ARGUMENT, "module was generated without the record kernels");
     long long g = grid;
     if (g <= 0) {
         int per_sm = 0;
@@ -644,7 +650,9 @@ extern "C" int cbx_adjoint_lanes(cbx_module* module, int block, long long* lanes
     if (!rc) rc = resolve_adjoint(module);
     if (rc) return rc;
     *lanes = 0;
+    if (!module->adj[2] || !module->adj[3]) return CBX_OK;
     for (int k = 2; k < 6; ++k) {
+        if (!module->adj[k]) continue;
         int per_sm = 0;
         rc = check_cu(g_drv.cuOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, module->adj[k], block, 0),
                       "cuOccupancyMaxActiveBlocksPerMultiprocessor");

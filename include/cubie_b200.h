@@ -158,7 +158,7 @@ int cbx_adjoint_launch_records(cbx_module* module, const cbx_solve_args* args, c
                                int phase, int block, int grid, void* stream);
 
 /* Runs that every kernel of the record form holds at once, a lane each, at this
- * block size. */
+ * block size; 0 for a module that was generated without them. */
 int cbx_adjoint_lanes(cbx_module* module, int block, long long* lanes);
 
 /* Size of the device scratch array behind cbx_solve_noalloc.  Every device

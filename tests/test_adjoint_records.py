@@ -234,6 +234,47 @@ def test_records_leave_room_for_the_caller(cuda_device, monkeypatch):
 
 
 @pytest.mark.gpu
+def test_modules_without_record_kernels_use_checkpoints(cuda_device):
+    """A cubin saved before there were record kernels: its checkpoint launches
+    run, a record launch is refused, the integrator takes checkpoints."""
+    import re
+    import torch
+    from cubie_b200 import _native
+    from cubie_b200.adjoint import AdjointIntegrator
+    s = _solver("fhn")
+    x0, p = (torch.tensor(v.astype(np.float32), device="cuda") for v in _batch("fhn", 40, 3))
+    want = AdjointIntegrator(s, record_share=0.0)
+    state, _, saved = want.forward(x0, p, 4.0)
+    grads = want.backward(saved, state)
+    prep = dict(saved["prep"])
+    header = (_native.DEVICE_INCLUDE / "cbx_adjoint.cuh").read_text()
+    macro = header[header.index("#define CBX_DEFINE_ADJOINT_KERNELS(CFG)"):]
+    first = macro[:macro.index('    extern "C" __global__ void CBX_LAUNCH_BOUNDS(CFG) cbx_adjoint_forward_records')]
+    first = first.rstrip().rstrip("\\").replace("ADJOINT_KERNELS", "TWO_ADJOINT_KERNELS", 1)
+    source, n = re.subn(r"CBX_DEFINE_ADJOINT_KERNELS\((.*)\)", lambda m: first + f"\nCBX_DEFINE_TWO_ADJOINT_KERNELS({m[1]})",
+                        prep["gen"].source)
+    assert n == 1
+    cubin, log = _native.compile_cubin(source, _native.default_options())
+    old = _native.Module(cubin, 0, log)
+    assert old.adjoint_lanes(128) == 0
+    key = next(k for k, v in s._prepared.items() if v is saved["prep"])
+    s._prepared[key] = dict(saved["prep"], module=old)
+    s._prepared[key].pop("record_lanes", None)
+    integ = AdjointIntegrator(s)
+    state2, _, saved2 = integ.forward(x0, p, 4.0)
+    assert saved2["records"] is None
+    for a, b in zip((state, *grads), (state2, *integ.backward(saved2, state))):
+        assert torch.equal(a, b)
+    adj = _native.AdjointArgs()
+    buf = torch.zeros((1 << 16,), device="cuda", dtype=torch.int32)
+    adj.seg = adj.ckpt_count = adj.step_count = buf.data_ptr()
+    adj.lane_words, adj.ckpt_every, adj.max_ckpts = 40, 1, 2
+    args = s.make_args(s._prepared[key], saved2["bufs"], x0, p, None, 40, 4.0, 0.0, 0.0)
+    with pytest.raises(_native.NativeError, match="without the record kernels"):
+        old.adjoint_launch(args, adj, 0, 128, records=True)
+
+
+@pytest.mark.gpu
 def test_free_bytes_follow_the_tensors(cuda_device):
     import torch
     from cubie_b200.adjoint import _free_bytes
